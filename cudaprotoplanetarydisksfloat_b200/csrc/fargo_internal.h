@@ -198,11 +198,12 @@ struct BatchDev {
   int accurate;              // precision mode of the batch's disks: which kernel set runs (FARGO_LAUNCHERS)
   int max_body;              // largest body count of the force sums (star + FeelDisk planets)
   // one-wave grids of the substep kernels (fargo_size_grids)
+  int any_corot;             // some disk's frame corotates: its planets come before the source terms
   int g_cfl, g_source1[4], g_potential, g_viscosity, g_source2[2], g_energy, g_velocities[2], g_transport;
 };
 
 // kernel entry points (kernels_step.cu), launched by fargo_api.cu
-#define FARGO_NKERNELS 14  // profiled slots per substep (boundary slots empty for rigid boundaries)
+#define FARGO_NKERNELS 15  // profiled slots per substep (boundary slots empty for rigid boundaries)
 #define FARGO_SEG_OUT 192  // largest azimuthal transport segment (output sectors per CTA)
 #define FARGO_BAND 8       // rings per transport CTA
 #define FARGO_RM_RINGS 8   // rings per ring-mean CTA (serial FP32 chain per ring)

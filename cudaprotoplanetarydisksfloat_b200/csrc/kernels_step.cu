@@ -9,11 +9,13 @@
 // device:
 //
 //   k_ring_mean<0>   serial FP32 ring means of v_theta for the CFL
-//   k_cfl_force      CFL minimum, disk-on-body forces on 4096-cell tiles; the
-//                    last block of each disk finishes the substep's scalar
-//                    work (dt, mass taper, potential parameters, planet kicks,
-//                    FP64 RK5, frame rotation, per-ring viscosity)
+//   k_cfl_force      CFL minimum, disk-on-body forces on 4096-cell tiles,
+//                    per-ring viscosity; the last block of each disk finishes
+//                    dt and the indirect term
 //   k_potential      star and planet potential of every cell
+//   k_planets        planet kicks, FP64 RK5, frame rotation, the next substep's
+//                    parameters: a branch of the graph beside the kernels below
+//                    (before them when the frame corotates)
 //   k_source1        Substep1 (pressure + potential + centrifugal kick) +
 //                    self-gravity kick; one instance per kind of disk
 //   k_viscosity      viscous stress tensor + velocity update + sub-Keplerian
@@ -44,6 +46,7 @@
 #include <algorithm>
 #include <cstdio>
 #include <type_traits>
+#include <vector>
 
 #include "fargo_internal.h"
 #include "fast_div.cuh"
@@ -356,6 +359,30 @@ __device__ void rotate_psys(DiskCtl* C, float angle) {
     yt = C->vy[i];
     C->vx[i] = xt * cost + yt * sint;
     C->vy[i] = -xt * sint + yt * cost;
+  }
+}
+
+// Arguments of the potential kernel: FillForcesArrays (Pframeforce.cu:49-61)
+// with the MassTaper of the substep (SourceEuler.cu:231-232), from the planets
+// at its start.
+__device__ void prepare_potential(const DiskDev& D, DiskCtl* C) {
+  const float PT = C->PhysicalTime;
+  float mt = PT / (D.MASSTAPER * 2.0 * M_PI);
+  mt = (mt > 1.0 ? 1.0 : pow(sin(mt * M_PI / 2.0), 2.0));
+  C->MassTaper = mt;
+  for (int k = 0; k < C->nb; k++) {
+    double xplanet = C->x[k], yplanet = C->y[k], mplanet = C->mass[k] * mt;
+    double PlanetDistance = sqrt(xplanet * xplanet + yplanet * yplanet);
+    double InvPlanetDistance3 = 1.0 / PlanetDistance / PlanetDistance / PlanetDistance;
+    double RRoche = PlanetDistance * pow((1.0 / 3.0 * mplanet), 1.0 / 3.0);
+    double smoothing = D.RocheSmoothing ? RRoche * D.ROCHESMOOTHING
+                                        : compute_smoothing(D, PlanetDistance, PT, C->PhysicalTimeInitial);
+    double smooth = smoothing * smoothing;
+    C->pxp[k] = (float)xplanet;
+    C->pyp[k] = (float)yplanet;
+    C->psmooth[k] = (float)smooth;
+    C->pmass[k] = (float)mplanet;
+    C->pipd3[k] = (float)InvPlanetDistance3;
   }
 }
 
@@ -681,28 +708,32 @@ __device__ float block_min_f(float v, float* sh) {
 
 // -------------------------------------------------------------- CFL + forces
 
-// The scalar part of the substep (SourceEuler.cu:231-264), run by the block
-// that completed a disk's last CFL tile (or, for a radial stripe, by
-// k_stripe_finish once every stripe's partials are gathered).
+// The scalar part of the substep (SourceEuler.cu:231-264) is split by what the
+// next kernels wait for:
+//  - finish_substep: the CFL minimum, dt and the indirect term (the disk's
+//    force on the star), run by the block that completes a disk's last CFL
+//    tile (or, for a radial stripe, by k_stripe_finish once every stripe's
+//    partials are gathered);
+//  - k_planets: the planet kicks, the FP64 planet integrator, the frame and the
+//    next substep's body and potential parameters, which nothing in this
+//    substep reads unless the frame corotates.
+// One block ran all of it in k_cfl_force before, with the rest of the GPU
+// waiting: cold code executed once per substep, 10 us on a 128x384 isothermal
+// disk and 57 us on a 1024x3072 adiabatic one with two live planets.
+// k_cfl_force 19.1 -> 11.7 us (128x384, one planet on a fixed orbit) and
+// 38.9 -> 14.1 us (256x768, two live planets); k_planets takes 9 and 25 us
+// beside the gas kernels.
 constexpr int kRkShared = 16;  // planets whose RK5 scratch fits in shared memory
-__device__ bool finish_serial(const DiskDev& D, DiskCtl* C, float newdt, const double* s_sum);
-__device__ void finish_serial_tail(const DiskDev& D, DiskCtl* C);
 
 // ConditionCFL host part (SourceEuler.cu:513-535): the shear limit DT1D
-// (ConditionCFLKernel2D2, Kernels.cu:1425-1428) of the ring pairs (i, i+1),
-// i in [i0, i1), folded into a thread's running minimum.
-__device__ __forceinline__ float dt1d_min(const DiskDev& D, int i0, int i1, int tid, int nt, float m) {
-#pragma unroll 4
-  for (int i = i0 + tid; i < i1; i += nt) {
-    float dt1 = 2.0 * PI_D * CFLSEC / (float)D.nsec / fabsf(D.vmoy[i] * D.invRmed[i] - D.vmoy[i + 1] * D.invRmed[i + 1]);
-    if (dt1 < m) m = dt1;
-  }
-  return m;
+// (ConditionCFLKernel2D2, Kernels.cu:1425-1428) of the ring pair (i, i+1).
+__device__ __forceinline__ float dt1d(const DiskDev& D, int i) {
+  return 2.0 * PI_D * CFLSEC / (float)D.nsec / fabsf(D.vmoy[i] * D.invRmed[i] - D.vmoy[i + 1] * D.invRmed[i + 1]);
 }
 
 // Inputs of the finishing sums of a whole disk: its CFL tiles' minima and
 // force partials ([sum][tile]), written by the blocks of this launch (read
-// through L2), and the shear limit of every ring pair.
+// through L2).
 struct DiskTiles {
   const DiskDev& D;
   int nct;
@@ -713,7 +744,7 @@ struct DiskTiles {
       float v = __ldcg(D.ringmin + t);
       if (v < m) m = v;
     }
-    return dt1d_min(D, 0, D.nrad - 1, tid, nt, m);
+    return m;
   }
   __device__ int ntiles() const { return nct; }
   __device__ double partial(int q, int t) const { return __ldcg(D.partials + (size_t)q * nct + t); }
@@ -754,83 +785,47 @@ struct StripeBlocks {
   }
 };
 
-// Substep scalars of one disk, run by one block: the CFL minimum, the disk
-// forces summed over the tiles in a fixed order, the viscosity per ring and
-// the serial part (on a shared-memory copy of the disk's control block, sC,
-// written back at the end).
-template <int NB, class Src>
-__device__ void finish_cfl_and_planets(const DiskDev& D, DiskCtl* Cg, DiskCtl* sC, float* shf, double* s_sum,
-                                       double* s_work, const Src& src) {
-  const int nrad = D.nrad, tid = threadIdx.x;
-  const int nct = src.ntiles();
-  float newdt = block_min_f(src.thread_min(tid, blockDim.x), shf);
-  // disk-force sums over the tiles in a fixed order: every thread a strided
-  // share of the tiles for all sums at once, the warps by shuffle, then the
-  // warps in order (s_work is free until the planet update)
-  const int nbody = min(Cg->nbody, NB), nsum = 4 * nbody;
-  const int w = tid >> 5, l = tid & 31, nw = blockDim.x >> 5;
-  double acc[4 * NB];
-#pragma unroll
-  for (int q = 0; q < 4 * NB; q++) acc[q] = 0.0;
-#pragma unroll 2
-  for (int t = tid; t < nct; t += blockDim.x) {
-#pragma unroll
-    for (int q = 0; q < 4 * NB; q++)
-      if (q < nsum) acc[q] += src.partial(q, t);
-  }
-#pragma unroll
-  for (int q = 0; q < 4 * NB; q++) {
-    if (q < nsum) {
-      const double v = warp_sum_d(acc[q]);
-      if (l == 0) s_work[q * nw + w] = v;
-    }
-  }
-  __syncthreads();
-  if (tid < nsum) {
-    double acc = 0.0;
-    for (int u = 0; u < nw; u++) acc += s_work[tid * nw + u];
-    s_sum[tid] = acc;
-  }
-  // FViscosity per ring for this substep (Viscosity.cu:84-85, SourceEuler.cu:350)
-  const float PT = Cg->PhysicalTime;
-  for (int i = tid; i < nrad; i += blockDim.x) D.visc[i] = fviscosity_ring(D, i, PT, Cg->PhysicalTimeInitial);
-  {
-    const int* src = reinterpret_cast<const int*>(Cg);
-    int* dst = reinterpret_cast<int*>(sC);
-    for (int k = tid; k < (int)(sizeof(DiskCtl) / 4); k += blockDim.x) dst[k] = src[k];
-  }
-  __syncthreads();
-  // the serial part on thread 0, the planet integrator on warp 0, the rest
-  // on thread 0 again
-  __shared__ int s_go;
-  if (tid == 0) s_go = finish_serial(D, sC, newdt, s_sum) ? 1 : 0;
-  __syncthreads();
-  if (s_go && tid < 32)
-    advance_system_rk5(D, sC, sC->dtf, sC->PhysicalTime, sC->nb <= kRkShared ? s_work : D.rk_work, tid);
-  __syncthreads();
-  if (s_go && tid == 0) finish_serial_tail(D, sC);
-  __syncthreads();
-  {
-    const int* src = reinterpret_cast<const int*>(sC);
-    int* dst = reinterpret_cast<int*>(Cg);
-    for (int k = tid; k < (int)(sizeof(DiskCtl) / 4); k += blockDim.x) dst[k] = src[k];
-  }
+// One force sum over the tiles in a fixed order: every thread a strided share,
+// the warps by shuffle into s_part[warp]; the caller adds the warps in order.
+template <class Src>
+__device__ __forceinline__ void tile_sum(const Src& src, int q, int nct, double* s_part) {
+  double acc = 0.0;
+#pragma unroll 4
+  for (int t = threadIdx.x; t < nct; t += blockDim.x) acc += src.partial(q, t);
+  acc = warp_sum_d(acc);
+  if ((threadIdx.x & 31) == 0) s_part[threadIdx.x >> 5] = acc;
+}
+__device__ __forceinline__ double warps_in_order(const double* s_part) {
+  double acc = 0.0;
+  for (int u = 0; u < (int)(blockDim.x >> 5); u++) acc += s_part[u];
+  return acc;
 }
 
-// ... through AdvanceSystemFromDisk; false: the DT stopped (non-finite or
-// non-positive CFL step), nothing more to do
-__device__ bool finish_serial(const DiskDev& D, DiskCtl* C, float newdt, const double* s_sum) {
-  const int nbody = C->nbody;
-  const float PT = C->PhysicalTime;
-  double DTd = (double)D.DT;
-  // MassTaper, SourceEuler.cu:231-232
-  float mt = PT / (D.MASSTAPER * 2.0 * M_PI);
-  mt = (mt > 1.0 ? 1.0 : pow(sin(mt * M_PI / 2.0), 2.0));
-  C->MassTaper = mt;
+// dt, the substep's bookkeeping and the indirect term, by one block (thread 0
+// does the scalar part on the control block in global memory).  shf: 32
+// floats, s_part: 2 x 32 doubles of shared memory.
+template <class Src>
+__device__ void finish_substep(const DiskDev& D, DiskCtl* C, float* shf, double (*s_part)[32], const Src& src) {
+  const int tid = threadIdx.x, w = tid >> 5, l = tid & 31;
+  const int nct = src.ntiles();
+  double dtemp = 0.0, dt = 0.0;
+  float PT = 0.0f;
+  int nsub = 0;
+  if (tid == 0) dtemp = C->dtemp, dt = C->dt, PT = C->PhysicalTime, nsub = C->nsub;
+  float m = warp_min_f(src.thread_min(tid, blockDim.x));
+  if (l == 0) shf[w] = m;
+  // the star's force sums are the outer ones (no ring lies inside radius 0)
+  tile_sum(src, 1, nct, s_part[0]);
+  tile_sum(src, 3, nct, s_part[1]);
+  __syncthreads();
+  if (tid != 0) return;
+  float newdt = shf[0];
+  for (int u = 1; u < (int)(blockDim.x >> 5); u++)
+    if (shf[u] < newdt) newdt = shf[u];
+  const double DTd = (double)D.DT;
   // substep count and dt (SourceEuler.cu:236-241, 535)
-  double dt = C->dt;
-  if (D.IsDisk && (!D.SloppyCFL || C->nsub == 0)) {
-    float DeltaT = DTd - C->dtemp;
+  if (D.IsDisk && (!D.SloppyCFL || nsub == 0)) {
+    float DeltaT = DTd - dtemp;
     if (DeltaT < newdt) newdt = DeltaT;
     float q = DeltaT / newdt;
     if (!(newdt > 0.0f) || !(q < 1.0e5f)) {
@@ -838,86 +833,130 @@ __device__ bool finish_serial(const DiskDev& D, DiskCtl* C, float newdt, const d
       C->more = 0;
       C->active = 0;
       C->counter = 0;
-      return false;
+      return;
     }
     int n = (int)ceilf(q);
-    dt = (DTd - C->dtemp) / (double)n;
-  } else if (!D.IsDisk && C->nsub == 0) {
+    dt = (DTd - dtemp) / (double)n;
+  } else if (!D.IsDisk && nsub == 0) {
     dt = DTd;
   }
+  dtemp += dt;
   C->dt = dt;
   C->dtf = (float)dt;
-  C->dtemp += dt;
-  if (C->nsub < FARGO_MAXLOG) D.log_dt[C->nsub] = dt;
-  float dtf = (float)dt;
-  if (D.Corotating) get_psys_info(D, C, 1);
+  C->dtemp = dtemp;
+  if (nsub < FARGO_MAXLOG) D.log_dt[nsub] = dt;
   // DiskOnPrimaryAcceleration (ComputeAccel for the star, SideEuler.cu:151-164):
-  // the Force fields are floats, their sum is a float.
+  // the Force fields are floats, their sum is a float; ComputeIndirectTerm,
+  // Pframeforce.cu:27-35
   float ax = 0.0f, ay = 0.0f;
   if (D.IsDisk) {
-    ax = (float)s_sum[0] + (float)s_sum[1];
-    ay = (float)s_sum[2] + (float)s_sum[3];
+    ax = 0.0f + (float)warps_in_order(s_part[0]);
+    ay = 0.0f + (float)warps_in_order(s_part[1]);
   }
-  // ComputeIndirectTerm, Pframeforce.cu:27-35
-  C->itx = -ax;
-  C->ity = -ay;
-  if (!D.Indirect_Term) {
-    C->itx = 0.0f;
-    C->ity = 0.0f;
+  C->itx = D.Indirect_Term ? -ax : 0.0f;
+  C->ity = D.Indirect_Term ? -ay : 0.0f;
+  C->time_start = PT;
+  nsub++;
+  C->nsub = nsub;
+  C->nsub_total++;
+  int more = (dtemp < 0.999999999 * DTd) ? 1 : 0;
+  if (more && nsub >= D.max_sub) {
+    C->error = 2;
+    more = 0;
   }
-  // FillForcesArrays arguments (Pframeforce.cu:49-61)
-  for (int k = 0; k < C->nb; k++) {
-    double xplanet = C->x[k], yplanet = C->y[k], mplanet = C->mass[k] * mt;
-    double PlanetDistance = sqrt(xplanet * xplanet + yplanet * yplanet);
-    double InvPlanetDistance3 = 1.0 / PlanetDistance / PlanetDistance / PlanetDistance;
-    double RRoche = PlanetDistance * pow((1.0 / 3.0 * mplanet), 1.0 / 3.0);
-    double smoothing = D.RocheSmoothing ? RRoche * D.ROCHESMOOTHING
-                                        : compute_smoothing(D, PlanetDistance, PT, C->PhysicalTimeInitial);
-    double smooth = smoothing * smoothing;
-    C->pxp[k] = (float)xplanet;
-    C->pyp[k] = (float)yplanet;
-    C->psmooth[k] = (float)smooth;
-    C->pmass[k] = (float)mplanet;
-    C->pipd3[k] = (float)InvPlanetDistance3;
-  }
-  // AdvanceSystemFromDisk, Pframeforce.cu:68-92
-  if (D.IsDisk) {
-    for (int b = 1; b < nbody; b++) {
-      int k = C->body_planet[b];
-      float gx = (float)s_sum[4 * b] + (float)s_sum[4 * b + 1];
-      float gy = (float)s_sum[4 * b + 2] + (float)s_sum[4 * b + 3];
-      C->vx[k] += dtf * gx;
-      C->vy[k] += dtf * gy;
-      C->vx[k] += dtf * C->itx;
-      C->vy[k] += dtf * C->ity;
-    }
-  }
-  return true;
+  C->more = more;
+  C->domega = 0.0f;  // k_planets sets it in a corotating frame
+  C->counter = 0;
 }
 
-// The rest of the substep's scalars, after the planet integrator.
-__device__ void finish_serial_tail(const DiskDev& D, DiskCtl* C) {
-  const double dt = C->dt, DTd = (double)D.DT;
-  const float PT = C->PhysicalTime;
-  C->domega = 0.0f;
-  if (D.Corotating) {
-    double OmegaNew = get_psys_info(D, C, 0) / dt;
-    double domega = OmegaNew - C->OmegaFrame;
-    if (D.IsDisk) C->domega = (float)domega;
-    C->OmegaFrame = (float)OmegaNew;
+// AdvanceSystemFromDisk, the planet integrator, the frame rotation and the
+// next substep's parameters (Pframeforce.cu:68-157, SourceEuler.cu:253-264):
+// one block per disk inside its DT.  The integrator runs on the lanes of warp
+// 0, the rest on thread 0, on a shared-memory copy of the control block.  It
+// reads what finish_substep left and writes only the planets, the time, the
+// frame and the parameters of the next substep, so it may run beside the
+// substep's later kernels once k_potential has read this substep's
+// parameters; in a corotating frame k_source1 reads its domega and frame.
+__global__ void __launch_bounds__(kThreads) k_planets(BatchDev B) {
+  __shared__ DiskDev D;
+  __shared__ DiskCtl sC;
+  __shared__ double s_part[4 * FARGO_MAXBODY][kThreads / 32];
+  __shared__ double s_work[FARGO_RK_WORK(kRkShared)];
+  const int tid = threadIdx.x;
+  if ((int)blockIdx.x >= B.act[0]) return;
+  copy_words(&D, B.disks + B.act_disk[blockIdx.x], sizeof(DiskDev));
+  __syncthreads();
+  DiskCtl* Cg = D.ctl;
+  copy_words(&sC, Cg, sizeof(DiskCtl));
+  __syncthreads();
+  DiskCtl* C = &sC;
+  if (C->error == 1) return;  // the DT stopped at this substep
+  const int nbody = min(C->nbody, FARGO_MAXBODY);
+  // a radial stripe: k_stripe_finish left the sums over every stripe's tiles
+  const int nct = D.stripe ? 1 : fargo_cfl_tiles_own(D);
+  if (D.IsDisk)
+    for (int q = 4; q < 4 * nbody; q++) tile_sum(DiskTiles{D, nct}, q, nct, s_part[q]);
+  __syncthreads();
+  if (tid >= 32) return;
+  const float dtf = C->dtf, PT = C->time_start;
+  if (tid == 0) {
+    if (D.Corotating) get_psys_info(D, C, 1);
+    // AdvanceSystemFromDisk, Pframeforce.cu:68-92
+    if (D.IsDisk) {
+      for (int b = 1; b < nbody; b++) {
+        const int k = C->body_planet[b];
+        const double(*p)[kThreads / 32] = s_part + 4 * b;
+        const float gx = (float)warps_in_order(p[0]) + (float)warps_in_order(p[1]);
+        const float gy = (float)warps_in_order(p[2]) + (float)warps_in_order(p[3]);
+        C->vx[k] += dtf * gx;
+        C->vy[k] += dtf * gy;
+        C->vx[k] += dtf * C->itx;
+        C->vy[k] += dtf * C->ity;
+      }
+    }
   }
-  rotate_psys(C, (float)(C->OmegaFrame * dt));
-  C->time_start = PT;
-  C->PhysicalTime = PT + dt;
-  C->nsub++;
-  C->nsub_total++;
-  C->more = (C->dtemp < 0.999999999 * DTd) ? 1 : 0;
-  if (C->more && C->nsub >= D.max_sub) {
-    C->error = 2;
-    C->more = 0;
+  __syncwarp();
+  advance_system_rk5(D, C, dtf, PT, C->nb <= kRkShared ? s_work : D.rk_work, tid);
+  __syncwarp();
+  if (tid == 0) {
+    const double dt = C->dt;
+    if (D.Corotating) {
+      double OmegaNew = get_psys_info(D, C, 0) / dt;
+      double domega = OmegaNew - C->OmegaFrame;
+      if (D.IsDisk) Cg->domega = (float)domega;
+      C->OmegaFrame = (float)OmegaNew;
+      Cg->OmegaFrame = C->OmegaFrame;
+      Cg->Xplanet_mark = C->Xplanet_mark;
+      Cg->Yplanet_mark = C->Yplanet_mark;
+    }
+    rotate_psys(C, (float)(C->OmegaFrame * dt));
+    C->PhysicalTime = PT + dt;
+    Cg->PhysicalTime = C->PhysicalTime;
+    prepare_bodies(D, C);
+    prepare_potential(D, C);
+    Cg->nbody = C->nbody;
+    Cg->MassTaper = C->MassTaper;
   }
-  prepare_bodies(D, C);
-  C->counter = 0;
+  __syncwarp();
+  for (int k = tid; k < C->nb; k += 32) {
+    Cg->x[k] = C->x[k];
+    Cg->y[k] = C->y[k];
+    Cg->vx[k] = C->vx[k];
+    Cg->vy[k] = C->vy[k];
+    Cg->pxp[k] = C->pxp[k];
+    Cg->pyp[k] = C->pyp[k];
+    Cg->psmooth[k] = C->psmooth[k];
+    Cg->pmass[k] = C->pmass[k];
+    Cg->pipd3[k] = C->pipd3[k];
+  }
+  if (tid < C->nbody) {
+    Cg->body_planet[tid] = C->body_planet[tid];
+    Cg->bx[tid] = C->bx[tid];
+    Cg->by[tid] = C->by[tid];
+    Cg->brs[tid] = C->brs[tid];
+    Cg->brh[tid] = C->brh[tid];
+    Cg->ba[tid] = C->ba[tid];
+  }
 }
 
 // ConditionCFLKernel1D + ConditionCFLKernel2D1 + the cell minimum of
@@ -929,7 +968,7 @@ __device__ void finish_serial_tail(const DiskDev& D, DiskCtl* C) {
 // writes its minimum and its force partials (inner / outer by the ring of
 // each cell), so that the finishing sums run in a fixed order.  Each block
 // takes a contiguous run of tiles; the block that completes a disk's last
-// tile finishes the substep's scalar work.
+// tile finishes the scalar work that the next kernels need.
 // NB >= every disk's body count (star + FeelDisk planets): the per-thread
 // FP64 force accumulators are sized for it.
 static_assert(FARGO_CFL_TILE_SMALL == 4 * kThreads && FARGO_CFL_TILE % FARGO_CFL_TILE_SMALL == 0,
@@ -945,12 +984,10 @@ static_assert(CFLSEC == 0.5, "the CFL limit's reciprocal form needs CFLSECURITY 
 template <int NB>
 __global__ void __launch_bounds__(kThreads, NB <= 1 ? 3 : 2) k_cfl_force(BatchDev B) {
   __shared__ DiskDev sD;
-  __shared__ DiskCtl sC;
   __shared__ float s_b[5][NB];
   __shared__ float s_min[2][32];                     // double-buffered by tile parity
   __shared__ double s_red[2][4 * NB][kThreads / 32];
-  __shared__ double s_sum[4 * FARGO_MAXBODY];
-  __shared__ double s_work[FARGO_RK_WORK(kRkShared)];
+  __shared__ double s_part[2][32];
   __shared__ unsigned s_ticket;
   __shared__ int s_nbody;
   const int tid = threadIdx.x, w = tid >> 5, l = tid & 31;
@@ -978,7 +1015,7 @@ __global__ void __launch_bounds__(kThreads, NB <= 1 ? 3 : 2) k_cfl_force(BatchDe
     const int nct = fargo_cfl_tiles_own(sD);
     if (s_ticket + (unsigned)run == (unsigned)nct) {
       __threadfence();
-      finish_cfl_and_planets<NB>(sD, Cr, &sC, s_min[0], s_sum, s_work, DiskTiles{sD, nct});
+      finish_substep(sD, Cr, s_min[0], s_part, DiskTiles{sD, nct});
     }
     run = 0;
     __syncthreads();
@@ -1087,6 +1124,15 @@ __global__ void __launch_bounds__(kThreads, NB <= 1 ? 3 : 2) k_cfl_force(BatchDe
           }
         }
       };
+      // once per ring: the shear limit of the pair (i, i+1), and FViscosity for
+      // this substep (Viscosity.cu:84-85, SourceEuler.cu:350)
+      auto ring = [&](int i) {
+        if (i < nrad - 1) {
+          const float dt1 = dt1d(D, i);
+          if (dt1 < lmin) lmin = dt1;
+        }
+        if (!D.stripe) D.visc[i] = fviscosity_ring(D, i, D.ctl->PhysicalTime, D.ctl->PhysicalTimeInitial);
+      };
       auto ring_consts = [&](int ic, float (&rt)[8]) {
         rt[0] = D.Rsup[ic] - D.Rinf[ic];
         rt[1] = D.dxtheta[ic];
@@ -1119,6 +1165,7 @@ __global__ void __launch_bounds__(kThreads, NB <= 1 ? 3 : 2) k_cfl_force(BatchDe
           const float4 ST = __ldg(reinterpret_cast<const float4*>(D.sin_cell + j));
           float rt[8];
           ring_consts(i, rt);
+          if (j == 0) ring(i);
           cell(i, j, V0.x, VR0.x, DN.x, VRP.x, V0.y, CS.x, CT.x, ST.x, rt);
           cell(i, j + 1, V0.y, VR0.y, DN.y, VRP.y, V0.z, CS.y, CT.y, ST.y, rt);
           cell(i, j + 2, V0.z, VR0.z, DN.z, VRP.z, V0.w, CS.z, CT.z, ST.z, rt);
@@ -1169,6 +1216,7 @@ __global__ void __launch_bounds__(kThreads, NB <= 1 ? 3 : 2) k_cfl_force(BatchDe
             if (!ok[u]) continue;
             float rt[8];
             ring_consts(ci[u], rt);
+            if (cj[u] == 0) ring(ci[u]);
             cell(ci[u], cj[u], v0[u], vr0[u], dn[u], vrp[u], vtp[u], csv[u], cth[u], sth[u], rt);
           }
         }
@@ -1212,8 +1260,8 @@ __global__ void __launch_bounds__(kThreads, NB <= 1 ? 3 : 2) k_cfl_force(BatchDe
 // ----------------------------------------------------------- radial stripes
 
 // A radial stripe's block for the gather across stripes (StripeBlocks): the
-// minimum over its CFL tiles and over the shear limits of its own ring pairs
-// (i, i+1) (the disk's last ring has none), its tile count, its body count
+// minimum over its CFL tiles (the shear limits of its own ring pairs (i, i+1)
+// among them; the disk's last ring has none), its tile count, its body count
 // and its force partials [sum][tile].  One block; the stripe is disk 0 of
 // its batch.
 __global__ void __launch_bounds__(kThreads) k_stripe_block(BatchDev B, double* out) {
@@ -1221,12 +1269,7 @@ __global__ void __launch_bounds__(kThreads) k_stripe_block(BatchDev B, double* o
   const DiskDev& D = B.disks[0];
   const int tid = threadIdx.x;
   const int nct = fargo_cfl_tiles_own(D);
-  float m = 1e30f;
-  for (int t = tid; t < nct; t += blockDim.x) {
-    const float v = D.ringmin[t];
-    if (v < m) m = v;
-  }
-  m = dt1d_min(D, D.own_lo, D.own_hi < D.nrad ? D.own_hi : D.nrad - 1, tid, blockDim.x, m);
+  float m = DiskTiles{D, nct}.thread_min(tid, blockDim.x);
   m = block_min_f(m, shf);
   const int nbody = D.ctl->nbody;
   if (tid == 0) {
@@ -1239,16 +1282,16 @@ __global__ void __launch_bounds__(kThreads) k_stripe_block(BatchDev B, double* o
 
 // The substep scalars of a radial stripe from every stripe's block (the
 // same minimum and the same sums, in the same order, as the whole disk's
-// finishing block forms): every stripe runs it on the same blocks, so every
-// stripe takes the same dt, planet update and substep count.
+// finishing block and k_planets form): every stripe runs it on the same
+// blocks, so every stripe takes the same dt, planet update and substep count.
+// The force sums replace the stripe's own partials (already in its block) for
+// k_planets.
 constexpr int kMaxStripes = 256;
-template <int NB>
 __global__ void __launch_bounds__(kThreads) k_stripe_finish(BatchDev B, const double* blk, int nstripe, int stride) {
   __shared__ DiskDev sD;
-  __shared__ DiskCtl sC;
   __shared__ float shf[32];
-  __shared__ double s_sum[4 * FARGO_MAXBODY];
-  __shared__ double s_work[FARGO_RK_WORK(kRkShared)];
+  __shared__ double s_part[4 * FARGO_MAXBODY][kThreads / 32];
+  __shared__ double s_star[2][32];
   __shared__ int s_t0[kMaxStripes + 1];
   const int tid = threadIdx.x;
   copy_words(&sD, B.disks, sizeof(DiskDev));
@@ -1261,7 +1304,15 @@ __global__ void __launch_bounds__(kThreads) k_stripe_finish(BatchDev B, const do
     s_t0[nstripe] = t;
   }
   __syncthreads();
-  finish_cfl_and_planets<NB>(sD, sD.ctl, &sC, shf, s_sum, s_work, StripeBlocks{blk, nstripe, stride, s_t0});
+  const StripeBlocks src{blk, nstripe, stride, s_t0};
+  DiskCtl* C = sD.ctl;
+  const int nsum = 4 * min(C->nbody, FARGO_MAXBODY);
+  const float PT = C->PhysicalTime;
+  for (int i = tid; i < sD.nrad; i += blockDim.x) sD.visc[i] = fviscosity_ring(sD, i, PT, C->PhysicalTimeInitial);
+  for (int q = 4; q < nsum; q++) tile_sum(src, q, src.ntiles(), s_part[q]);
+  __syncthreads();
+  if (tid >= 4 && tid < nsum) sD.partials[tid] = warps_in_order(s_part[tid]);
+  finish_substep(sD, C, shf, s_star, src);
 }
 
 // ----------------------------------------------------------- source terms
@@ -2982,6 +3033,7 @@ __global__ void k_dt_begin(BatchDev B) {
     C->more = 1;
     C->counter = 0;
     prepare_bodies(D, C);
+    prepare_potential(D, C);
   }
   __syncthreads();
   compact_active(B);
@@ -3409,12 +3461,38 @@ void fargo_launch_cs_isothermal(const BatchDev& b, int only_disk, cudaStream_t s
 
 
 const char* fargo_substep_kernel_name(int k) {
-  static const char* names[] = {"k_ring_mean_cfl", "k_cfl_force",    "k_potential",  "k_boundary_0",
-                                "k_source1",       "k_viscosity",    "k_source2",    "k_boundary_1",
-                                "k_energy",        "k_ring_mean_tr", "k_transport",  "k_velocities",
-                                "k_boundary_2",    "k_substep_end"};
+  static const char* names[] = {"k_ring_mean_cfl", "k_cfl_force", "k_potential",    "k_planets",   "k_boundary_0",
+                                "k_source1",       "k_viscosity", "k_source2",      "k_boundary_1", "k_energy",
+                                "k_ring_mean_tr",  "k_transport", "k_velocities",   "k_boundary_2", "k_substep_end"};
   return (k >= 0 && k < FARGO_NKERNELS) ? names[k] : "";
 }
+
+// A side branch of a graph under capture, without a second stream: the nodes
+// launched between begin() and leave() become a branch, those after leave()
+// depend on what preceded begin(), and join() makes the next one depend on the
+// branch too.  begin() is false, and nothing happens, outside a capture.
+struct Branch {
+  cudaStream_t s = nullptr;
+  std::vector<cudaGraphNode_t> before, tip;
+  static bool nodes(cudaStream_t s, std::vector<cudaGraphNode_t>& v) {
+    cudaStreamCaptureStatus st;
+    const cudaGraphNode_t* deps = nullptr;
+    size_t n = 0;
+    if (cudaStreamGetCaptureInfo(s, &st, nullptr, nullptr, &deps, &n) != cudaSuccess) return false;
+    if (st != cudaStreamCaptureStatusActive) return false;
+    v.assign(deps, deps + n);
+    return true;
+  }
+  bool begin(cudaStream_t stream) {
+    s = stream;
+    return nodes(s, before);
+  }
+  void leave() {
+    nodes(s, tip);
+    cudaStreamUpdateCaptureDependencies(s, before.data(), before.size(), cudaStreamSetCaptureDependencies);
+  }
+  void join() { cudaStreamUpdateCaptureDependencies(s, tip.data(), tip.size(), cudaStreamAddCaptureDependencies); }
+};
 
 void fargo_launch_substep(const BatchDev& b, cudaGraphConditionalHandle h, int use_handle, cudaStream_t s,
                           int max_nsec, long long* launches, cudaEvent_t* ev, int part) {
@@ -3446,6 +3524,13 @@ void fargo_launch_substep(const BatchDev& b, cudaGraphConditionalHandle h, int u
   }
   REC();
   k_potential<<<b.g_potential, kThreads, 0, s>>>(b);
+  REC();
+  // inside a graph the planets run beside the rest of the substep, unless its
+  // kernels read the new frame
+  Branch branch;
+  const bool fork = !b.any_corot && branch.begin(s);
+  k_planets<<<b.ndisk, kThreads, 0, s>>>(b);
+  if (fork) branch.leave();
   REC();
   if (b.any_bc) {
     k_bc_rings<0><<<b.ring_grid, kThreads, 0, s>>>(b);
@@ -3484,6 +3569,7 @@ void fargo_launch_substep(const BatchDev& b, cudaGraphConditionalHandle h, int u
     k_bc_disk<<<b.ndisk, kThreads, 0, s>>>(b);
   }
   REC();
+  if (fork) branch.join();
   k_substep_end<<<1, kThreads, 0, s>>>(b, h, use_handle);
   REC();
 #undef REC
@@ -3496,14 +3582,7 @@ void fargo_launch_stripe_block(const BatchDev& b, double* out, cudaStream_t s) {
 
 int fargo_launch_stripe_finish(const BatchDev& b, const double* blk, int nstripe, int stride, cudaStream_t s) {
   if (nstripe < 1 || nstripe > kMaxStripes) return 1;
-  if (b.max_body <= 1)
-    k_stripe_finish<1><<<1, kThreads, 0, s>>>(b, blk, nstripe, stride);
-  else if (b.max_body <= 2)
-    k_stripe_finish<2><<<1, kThreads, 0, s>>>(b, blk, nstripe, stride);
-  else if (b.max_body <= 4)
-    k_stripe_finish<4><<<1, kThreads, 0, s>>>(b, blk, nstripe, stride);
-  else
-    k_stripe_finish<FARGO_MAXBODY><<<1, kThreads, 0, s>>>(b, blk, nstripe, stride);
+  k_stripe_finish<<<1, kThreads, 0, s>>>(b, blk, nstripe, stride);
   return 0;
 }
 
@@ -3552,13 +3631,13 @@ cudaError_t fargo_size_grids(BatchDev& b, int nsm, long long ncell_tiles, int ni
   return wave((const void*)k_transport<6>, kTT, fargo_transport_smem_bytes(1), nitems, &b.g_transport);
 }
 
-// Launches of one substep: 6 kernels, one Substep1 instance per kind of disk
+// Launches of one substep: 7 kernels, one Substep1 instance per kind of disk
 // present, the energy kernel when a disk is adiabatic, the isothermal and the
 // adiabatic forms of Substep2, transport and the velocity update when the
 // batch holds both, two per boundary call when a disk has a non-rigid
 // boundary.
 int fargo_substep_launches(const BatchDev& b) {
-  return 6 + __builtin_popcount((unsigned)b.src1_classes) + (b.ntheta_adi ? 1 : 0) +
+  return 7 + __builtin_popcount((unsigned)b.src1_classes) + (b.ntheta_adi ? 1 : 0) +
          3 * ((b.ntheta_iso && b.ntheta_adi) ? 2 : 1) + (b.any_bc ? 6 : 0);
 }
 
