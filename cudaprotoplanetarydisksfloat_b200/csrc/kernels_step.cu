@@ -624,16 +624,18 @@ __device__ __forceinline__ void qst(float* p, const Quad<V>& q, const float (&v)
 
 // -------------------------------------------------------------- reductions
 
-// DeviceReduce<float> (Kernels.cu:431-557) of f(0) .. f(n-1) in the
-// reference's order of operations, for the whole block (kThreads threads):
-// getNumBlocksAndThreads (Kernels.cu:404-429) picks the reference's block
-// count and size, each of its blocks is reduced in turn as deviceReduceKernel
-// does (Kernels.cu:269-383: the bounds-checked form, since IsPow2 is false
-// for every n > 1; shared-memory tree down to 64, the last warp by shuffles),
-// and the block sums are added in order as its host loop does.  Result in
-// every thread.  n > 128 (the reference launches no block below that).
-template <class F>
-__device__ float ref_device_reduce(F f, int n, float* sm) {
+// DeviceReduce<float> (Kernels.cu:431-557) of f(q, 0) .. f(q, n-1) for NQ
+// quantities q at once, each in the reference's order of operations, for the
+// whole block (kThreads threads): getNumBlocksAndThreads (Kernels.cu:404-429)
+// picks the reference's block count and size, each of its blocks is reduced in
+// turn as deviceReduceKernel does (Kernels.cu:269-383: the bounds-checked form,
+// since IsPow2 is false for every n > 1; shared-memory tree down to 64, the
+// last warp by shuffles), and the block sums are added in order as its host
+// loop does.  Results in every thread.  n > 128 (the reference launches no
+// block below that).  The quantities share the barriers, whose latency is the
+// whole cost.  sm: NQ * kThreads floats.
+template <int NQ, class F>
+__device__ void ref_device_reduce(F f, int n, float* sm, float (&res)[NQ]) {
   long np2 = 1;
   while (np2 < n) np2 <<= 1;
   const long maxBlocks = np2 / 256;
@@ -643,35 +645,52 @@ __device__ float ref_device_reduce(F f, int n, float* sm) {
   long blocks = (n + (2L * T - 1)) / (2L * T);
   if (blocks > maxBlocks) blocks = maxBlocks;
   const int t = threadIdx.x;
-  float total = 0.0f;
+  float total[NQ];
+#pragma unroll
+  for (int q = 0; q < NQ; q++) total[q] = 0.0f;
   for (long b = 0; b < blocks; b++) {
-    float my = 0.0f;
+    float my[NQ];
+#pragma unroll
+    for (int q = 0; q < NQ; q++) my[q] = 0.0f;
     __syncthreads();
     if (t < T) {
       const long gridSize = 2L * T * blocks;
       for (long i = b * 2L * T + t; i < n; i += gridSize) {
-        my += f(i);
-        if (i + T < n) my += f(i + T);
+#pragma unroll
+        for (int q = 0; q < NQ; q++) {
+          my[q] += f(q, i);
+          if (i + T < n) my[q] += f(q, i + T);
+        }
       }
-      sm[t] = my;
+#pragma unroll
+      for (int q = 0; q < NQ; q++) sm[q * kThreads + t] = my[q];
     }
     __syncthreads();
-    for (int stride = 256; stride >= 64; stride >>= 1) {
-      if (T >= 2 * stride && t < stride) sm[t] = my = my + sm[t + stride];
+    for (int stride = 128; stride >= 64; stride >>= 1) {
+      if (T >= 2 * stride && t < stride) {
+#pragma unroll
+        for (int q = 0; q < NQ; q++) sm[q * kThreads + t] = my[q] = my[q] + sm[q * kThreads + t + stride];
+      }
       __syncthreads();
     }
     if (t < 32) {
-      if (T >= 64) my = my + sm[t + 32];
-      for (int off = 16; off > 0; off >>= 1) my += __shfl_down_sync(0xffffffffu, my, off);
-      if (t == 0) total += my;
+#pragma unroll
+      for (int q = 0; q < NQ; q++) {
+        if (T >= 64) my[q] = my[q] + sm[q * kThreads + t + 32];
+        for (int off = 16; off > 0; off >>= 1) my[q] += __shfl_down_sync(0xffffffffu, my[q], off);
+        if (t == 0) total[q] += my[q];
+      }
     }
   }
   __syncthreads();
-  if (t == 0) sm[0] = total;
+  if (t == 0) {
+#pragma unroll
+    for (int q = 0; q < NQ; q++) sm[q] = total[q];
+  }
   __syncthreads();
-  const float r = sm[0];
+#pragma unroll
+  for (int q = 0; q < NQ; q++) res[q] = sm[q];
   __syncthreads();
-  return r;
 }
 
 __device__ __forceinline__ double warp_sum_d(double v) {
@@ -3002,8 +3021,9 @@ __global__ void k_substep_end(BatchDev B, cudaGraphConditionalHandle h, int use_
     for (int d = 0; d < B.ndisk; d++) {
       const DiskDev& D = B.disks[d];
       if (!D.OpenInner || !D.IsDisk || !D.ctl->active) continue;  // block-uniform
-      const float lost = ref_device_reduce([&](long j) { return D.lost[j]; }, D.nsec, sm);
-      if (threadIdx.x == 0) D.ctl->LostMass += lost;
+      float lost[1];
+      ref_device_reduce<1>([&](int, long j) { return D.lost[j]; }, D.nsec, sm, lost);
+      if (threadIdx.x == 0) D.ctl->LostMass += lost[0];
     }
     __syncthreads();
   }
@@ -3100,183 +3120,309 @@ __global__ void k_cs_ringmean(BatchDev B, int only_disk) {
 
 // ------------------------------------------------------- boundary conditions
 
-// ApplyBoundaryCondition (SideEuler.cu:172-182), ring-local part, one block
-// per ring of the disks inside their DT (contiguous runs, DiskDev in shared
-// memory):
-//  - NONREFLECTING, adiabatic: ComputeSoundSpeed first (SideEuler.cu:176-177),
-//    then, for alpha viscosity, the ring-mean sound speed and the viscosity
-//    that the next ComputeViscousTerms rebuilds from it (Viscosity.cu:79-86);
-//  - EVANESCENT: EvanescentBoundaryKernel (Kernels.cu:1076-1124) in the
-//    damping zones; at the first call of a substep it is preceded by
-//    CorrectVtheta, applied here in place (k_source1 then skips it).
-// stage 0, 1, 2: the calls before Substep1, before Substep3, after Transport
-// (SourceEuler.cu:267, 285, 292).
-template <int stage>
-__global__ void __launch_bounds__(kThreads) k_bc_rings(BatchDev B) {
-  __shared__ DiskDev sD;
+// ApplyBoundaryCondition (SideEuler.cu:172-182), edge-ring part, by one block:
+// OpenBoundaryKernel (Kernels.cu:623-637) and NonReflectingBoundary
+// (SideEuler.cu:70-101: ReduceCs, the angular offsets i_angle / i_angle2,
+// NonReflectingBoundaryKernel, ReduceMean, MinusMeanKernel,
+// Kernels.cu:640-722), with the ring means reduced in DeviceReduce's order.
+// The sound speed may have been written by other blocks of this launch: it is
+// read through L2.  sm: 4 * kThreads floats.
+__device__ void boundary_edges(const DiskDev& D, float* sm) {
+  __shared__ int s_angle[2];
   const int tid = threadIdx.x;
-  const int na = B.act[0];
-  const int ntile = na > 0 ? B.act_ring_off[na] : 0;
-  const int per = (ntile + gridDim.x - 1) / gridDim.x;
-  const int t0 = blockIdx.x * per, t1 = min(t0 + per, ntile);
-  int lo = 0, hi = -1;
-  for (int t = t0; t < t1; t++) {
-    if (t >= hi) {  // block-uniform: entering a disk
-      const int a = find_range(B.act_ring_off, na, t);
-      lo = B.act_ring_off[a];
-      hi = B.act_ring_off[a + 1];
-      __syncthreads();
-      copy_words(&sD, B.disks + B.act_disk[a], sizeof(DiskDev));
-      __syncthreads();
+  const int nsec = D.nsec, nrad = D.nrad;
+  float* Dn = D.dens;
+  float* En = D.energy;
+  float* Vr = D.vrad;
+  if (D.OpenInner) {
+    const float SigmaMed = D.SigmaMed[0];
+    for (int j = tid; j < nsec; j += kThreads) {
+      const int i = 1;
+      Dn[(i - 1) * nsec + j] = Dn[i * nsec + j];
+      En[(i - 1) * nsec + j] = En[i * nsec + j];
+      if (Vr[(i + 1) * nsec + j] > 0.0 || (Dn[i * nsec + j] < SigmaMed))
+        Vr[i * nsec + j] = 0.0;
+      else
+        Vr[i * nsec + j] = Vr[(i + 1) * nsec + j];
     }
-    const DiskDev& D = sD;
-    const DiskCtl* C = D.ctl;
-    if (!D.IsDisk) continue;
-    const int i = t - lo, nsec = D.nsec;
-    const size_t r0 = (size_t)i * nsec;
-    if (D.NonReflecting && D.Adiabatic) {
-      for (int j = tid; j < nsec; j += kThreads)
-        D.cs[r0 + j] = sqrtf(D.ADIABATICINDEX * (D.ADIABATICINDEX - 1.0) * D.energy[r0 + j] / D.dens[r0 + j]);
-      if (D.ViscosityAlpha) {
-        __syncthreads();
-        if (tid == 0) {
-          float sum = 0.0f;  // Make1DprofileKernel: sectors in order
-          if (D.accurate) {
-            KahanSum ks;
-            for (int j = 0; j < nsec; j++) ks.add(D.cs[r0 + j]);
-            sum = ks.s;
-          } else {
-            for (int j = 0; j < nsec; j++) sum += D.cs[r0 + j];
-          }
-          D.csmean[i] = sum / (float)nsec;
-          D.visc[i] = fviscosity_ring(D, i, C->time_start, C->PhysicalTimeInitial);
-        }
+  }
+  if (D.NonReflecting) {
+    const int rings[4] = {0, 1, nrad - 1, nrad - 2};
+    auto cs_at = [&](int r, int j) -> float {
+      return D.Adiabatic ? __ldcg(D.cs + (size_t)r * nsec + j) : D.cs_ring[r];
+    };
+    float cm[4];
+    ref_device_reduce<4>([&](int q, long j) -> float { return cs_at(rings[q], (int)j); }, nsec, sm, cm);
+    if (tid == 0) {
+      const float cs0_r = cm[0] / (float)nsec, cs1_r = cm[1] / (float)nsec;
+      const float csnrm1_r = cm[2] / (float)nsec, csnrm2_r = cm[3] / (float)nsec;
+      // host arithmetic of NonReflectingBoundary, pow() of the radii from the host
+      double dangle = (D.nr_pow_in - 1.0) / (.5 * (cs0_r + cs1_r));
+      dangle *= (D.Rmed[1] - D.Rmed[0]);
+      s_angle[0] = (int)(dangle / 2.0 / PI_D * (float)nsec + .5);
+      double dangle2 = (D.nr_pow_out - 1.0) / (.5 * (csnrm1_r + csnrm2_r));
+      dangle2 *= (D.Rmed[nrad - 1] - D.Rmed[nrad - 2]);
+      s_angle[1] = (int)(dangle2 / 2.0 / PI_D * (float)nsec + .5);
+    }
+    __syncthreads();
+    const int i_angle = s_angle[0], i_angle2 = s_angle[1];
+    const float SigmaMed = D.SigmaMed[1], SigmaMed2 = D.SigmaMed[nrad - 2];
+    // Rings 1, 2 and NRAD-2 are read, rings 0, 1 (v_r) and NRAD-1 written: the
+    // samples of four sectors are loaded before any is stored.  On a grid so
+    // coarse that an offset exceeds a turn, the one wrap of the reference leaves
+    // its target in the next ring, which other sectors read or write: those
+    // offsets keep the sectors in order, one at a time.
+    const int i1 = nsec, iq = (nrad - 2) * nsec, io = (nrad - 1) * nsec;
+    const bool in_ring = abs(i_angle) <= nsec && abs(i_angle2) <= nsec;
+    for (int j = tid; !in_ring && j < nsec; j += kThreads) {
+      int jp = j + i_angle;
+      if (jp >= nsec) jp -= nsec;
+      if (jp < 0) jp += nsec;
+      Dn[jp] = Dn[i1 + j];
+      En[jp] = En[i1 + j];
+      float Vrad_med = -cs_at(1, j) * (Dn[i1 + j] - SigmaMed) / SigmaMed;
+      Vr[i1 + j] = 2. * Vrad_med - Vr[i1 + nsec + j];
+      jp = j - i_angle2;
+      if (jp >= nsec) jp -= nsec;
+      if (jp < 0) jp += nsec;
+      Dn[io + j] = Dn[iq + jp];
+      En[io + j] = En[iq + jp];
+      Vrad_med = cs_at(nrad - 1, j) * (Dn[iq + j] - SigmaMed2) / SigmaMed2;
+      Vr[io + j] = 2. * Vrad_med - Vr[iq + j];
+    }
+    for (int j0 = tid; in_ring && j0 < nsec; j0 += 4 * kThreads) {
+      float d1[4], e1[4], v2[4], c1[4], co[4], dq[4], ds[4], es[4], vq[4];
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        const int j = min(j0 + u * kThreads, nsec - 1);
+        int jp = j - i_angle2;
+        if (jp >= nsec) jp -= nsec;
+        if (jp < 0) jp += nsec;
+        d1[u] = Dn[i1 + j];
+        e1[u] = En[i1 + j];
+        v2[u] = Vr[i1 + nsec + j];
+        c1[u] = cs_at(1, j);
+        co[u] = cs_at(nrad - 1, j);
+        dq[u] = Dn[iq + j];
+        ds[u] = Dn[iq + jp];
+        es[u] = En[iq + jp];
+        vq[u] = Vr[iq + j];
+      }
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        const int j = j0 + u * kThreads;
+        if (j >= nsec) break;
+        int jp = j + i_angle;
+        if (jp >= nsec) jp -= nsec;
+        if (jp < 0) jp += nsec;
+        Dn[jp] = d1[u];
+        En[jp] = e1[u];
+        float Vrad_med = -c1[u] * (d1[u] - SigmaMed) / SigmaMed;
+        Vr[i1 + j] = 2. * Vrad_med - v2[u];
+        Dn[io + j] = ds[u];
+        En[io + j] = es[u];
+        Vrad_med = co[u] * (dq[u] - SigmaMed2) / SigmaMed2;
+        Vr[io + j] = 2. * Vrad_med - vq[u];
       }
     }
-    if (D.Evanescent) {
-      const float Rm = D.Rmed[i];
-      if (stage == 0 && C->domega != 0.0f)
-        for (int j = tid; j < nsec; j += kThreads) D.vtheta[r0 + j] = D.vtheta[r0 + j] - C->domega * Rm;
-      const float DRMIN = D.ev_DRMIN, DRMAX = D.ev_DRMAX;
-      if ((Rm < DRMIN) || (Rm > DRMAX)) {
-        float damping, lambda = 0.0f;
-        if (Rm < DRMIN) {
-          damping = (Rm - DRMIN) / (D.Rmed[0] - DRMIN);
-          lambda = damping * damping * 10.0 * C->dtf / D.ev_Tin;
-        }
-        if (Rm > DRMAX) {
-          damping = (Rm - DRMAX) / (D.Rmed[D.nrad - 1] - DRMAX);
-          lambda = damping * damping * 10.0 * C->dtf / D.ev_Tout;
-        }
-        // the self-gravity form subtracts Rmed * GLOBAL_bufarray_d[i], an
-        // array the reference never fills (zero)
-        const float AspectRatio = aspect_ratio_dev(D, Rm, C->time_start, C->PhysicalTimeInitial);
-        float vtheta0 = sqrtf(1.0 * 1.0 / Rm *
-                              (1.0 - (1.0 + D.SIGMASLOPE - 2.0 * D.FLARINGINDEX) * powf(AspectRatio, 2.0f) *
-                                         powf(Rm, (float)(2.0 * D.FLARINGINDEX))));
-        vtheta0 -= Rm * C->OmegaFrame;
-        const float vrad0 = -3.0 * D.visc[i] / Rm * (-D.SIGMASLOPE + .5);
-        const float dens0 = D.SigmaMed[i];
-        const float energy0 = D.EnergyMed[i];
-        for (int j = tid; j < nsec; j += kThreads) {
-          const size_t l = r0 + j;
-          D.vrad[l] = (D.vrad[l] + lambda * vrad0) / (1.0 + lambda);
-          D.vtheta[l] = (D.vtheta[l] + lambda * vtheta0) / (1.0 + lambda);
-          D.dens[l] = (D.dens[l] + lambda * dens0) / (1.0 + lambda);
-          if (D.Adiabatic) D.energy[l] = (D.energy[l] + lambda * energy0) / (1.0 + lambda);
-        }
+    __syncthreads();
+    const size_t lo = (size_t)(nrad - 1) * nsec;
+    float me[4];
+    ref_device_reduce<4>([&](int q, long j) -> float { return (q < 2 ? Dn : En)[(q & 1) ? lo + j : j]; }, nsec, sm, me);
+    const float mean_dens_r = me[0] / (float)nsec, mean_dens_r2 = me[1] / (float)nsec;
+    const float mean_energy_r = me[2] / (float)nsec, mean_energy_r2 = me[3] / (float)nsec;
+    const float sm0 = D.SigmaMed[0], sm1 = D.SigmaMed[nrad - 1];
+    const float em0 = D.EnergyMed[0], em1 = D.EnergyMed[nrad - 1];
+    for (int j0 = tid; j0 < nsec; j0 += 2 * kThreads) {
+      float v[2][4];
+#pragma unroll
+      for (int u = 0; u < 2; u++) {
+        const int j = min(j0 + u * kThreads, nsec - 1);
+        v[u][0] = Dn[j], v[u][1] = En[j], v[u][2] = Dn[lo + j], v[u][3] = En[lo + j];
+      }
+#pragma unroll
+      for (int u = 0; u < 2; u++) {
+        const int j = j0 + u * kThreads;
+        if (j >= nsec) break;
+        Dn[j] = v[u][0] + (sm0 - mean_dens_r);
+        En[j] = v[u][1] + (em0 - mean_energy_r);
+        Dn[lo + j] = v[u][2] + (sm1 - mean_dens_r2);
+        En[lo + j] = v[u][3] + (em1 - mean_energy_r2);
       }
     }
   }
 }
 
-// ApplyBoundaryCondition, edge-ring part, one block per disk inside its DT:
-// OpenBoundaryKernel (Kernels.cu:623-637) and NonReflectingBoundary
-// (SideEuler.cu:70-101: ReduceCs, the angular offsets i_angle / i_angle2,
-// NonReflectingBoundaryKernel, ReduceMean, MinusMeanKernel,
-// Kernels.cu:640-722), with the ring means reduced in DeviceReduce's order.
-__global__ void __launch_bounds__(kThreads) k_bc_disk(BatchDev B) {
-  __shared__ float sm[kThreads];
-  __shared__ int s_angle[2];
+// x / d in double from r = RN(1/d) (Markstein's method as in div_by_recip):
+// the correctly rounded quotient for normal operands, in three operations.
+__device__ __forceinline__ double div_by_recip_d(double x, double d, double r) {
+  const double q0 = __dmul_rn(x, r);
+  return __fma_rn(__fma_rn(-q0, d, x), r, q0);
+}
+
+// ApplyBoundaryCondition (SideEuler.cu:172-182) of the disks inside their DT,
+// one launch: a block per ring (contiguous runs, DiskDev in shared memory), and
+// the edge rings by the block that completes a disk's last ring.
+//  - NONREFLECTING, adiabatic: ComputeSoundSpeed first (SideEuler.cu:176-177),
+//    then, for alpha viscosity, the ring-mean sound speed and the viscosity
+//    that the next ComputeViscousTerms rebuilds from it (Viscosity.cu:79-86):
+//    the mean is one chain of NSEC ordered additions, run from shared memory;
+//  - EVANESCENT: EvanescentBoundaryKernel (Kernels.cu:1076-1124) in the
+//    damping zones; at the first call of a substep it is preceded by
+//    CorrectVtheta, applied here in place (k_source1 then skips it);
+//  - OPEN and NONREFLECTING: boundary_edges.
+// stage 0, 1, 2: the calls before Substep1, before Substep3, after Transport
+// (SourceEuler.cu:267, 285, 292).
+// Latency-bound (a few rings of L2-resident data, barriers, one chain of
+// additions).  Against two launches with one global load at a time, one
+// reduction at a time and an FP64 division per damped value: NONREFLECTING
+// 256x768 36 -> 16.5 us, EVANESCENT 384x1152 17.4 -> 5.7 us per call.
+constexpr int kBcCols = 1024;  // sectors of a ring staged at a time
+template <int stage>
+__global__ void __launch_bounds__(kThreads) k_boundary(BatchDev B) {
+  __shared__ DiskDev sD;
+  __shared__ __align__(16) float s_row[kBcCols];
+  static_assert(kBcCols == 4 * kThreads, "the reductions' scratch");
+  __shared__ unsigned s_ticket;
   const int tid = threadIdx.x;
   const int na = B.act[0];
-  for (int a = blockIdx.x; a < na; a += gridDim.x) {
-    const DiskDev& D = B.disks[B.act_disk[a]];
-    if (!D.IsDisk || !(D.OpenInner || D.NonReflecting)) continue;
-    const int nsec = D.nsec, nrad = D.nrad;
-    float* Dn = D.dens;
-    float* En = D.energy;
-    float* Vr = D.vrad;
-    if (D.OpenInner) {
-      const float SigmaMed = D.SigmaMed[0];
-      for (int j = tid; j < nsec; j += kThreads) {
-        const int i = 1;
-        Dn[(i - 1) * nsec + j] = Dn[i * nsec + j];
-        En[(i - 1) * nsec + j] = En[i * nsec + j];
-        if (Vr[(i + 1) * nsec + j] > 0.0 || (Dn[i * nsec + j] < SigmaMed))
-          Vr[i * nsec + j] = 0.0;
-        else
-          Vr[i * nsec + j] = Vr[(i + 1) * nsec + j];
-      }
-    }
-    if (D.NonReflecting) {
-      auto csr = [&](int r) {
-        return [&, r](long j) -> float {
-          return D.Adiabatic ? D.cs[(size_t)r * nsec + j] : D.cs_ring[r];
-        };
-      };
-      const float cs0_r = ref_device_reduce(csr(0), nsec, sm) / (float)nsec;
-      const float cs1_r = ref_device_reduce(csr(1), nsec, sm) / (float)nsec;
-      const float csnrm1_r = ref_device_reduce(csr(nrad - 1), nsec, sm) / (float)nsec;
-      const float csnrm2_r = ref_device_reduce(csr(nrad - 2), nsec, sm) / (float)nsec;
-      if (tid == 0) {
-        // host arithmetic of NonReflectingBoundary, pow() of the radii from the host
-        double dangle = (D.nr_pow_in - 1.0) / (.5 * (cs0_r + cs1_r));
-        dangle *= (D.Rmed[1] - D.Rmed[0]);
-        s_angle[0] = (int)(dangle / 2.0 / PI_D * (float)nsec + .5);
-        double dangle2 = (D.nr_pow_out - 1.0) / (.5 * (csnrm1_r + csnrm2_r));
-        dangle2 *= (D.Rmed[nrad - 1] - D.Rmed[nrad - 2]);
-        s_angle[1] = (int)(dangle2 / 2.0 / PI_D * (float)nsec + .5);
-      }
-      __syncthreads();
-      const int i_angle = s_angle[0], i_angle2 = s_angle[1];
-      const float* cs = D.cs;
-      const float SigmaMed = D.SigmaMed[1], SigmaMed2 = D.SigmaMed[nrad - 2];
-      for (int j = tid; j < nsec; j += kThreads) {
-        int i = 1, jp = j + i_angle;
-        if (jp >= nsec) jp -= nsec;
-        if (jp < 0) jp += nsec;
-        float csv = D.Adiabatic ? cs[(size_t)i * nsec + j] : D.cs_ring[i];
-        Dn[jp] = Dn[i * nsec + j];
-        En[jp] = En[i * nsec + j];
-        float Vrad_med = -csv * (Dn[i * nsec + j] - SigmaMed) / SigmaMed;
-        Vr[i * nsec + j] = 2. * Vrad_med - Vr[(i + 1) * nsec + j];
-        i = nrad - 1;
-        jp = j - i_angle2;
-        if (jp >= nsec) jp -= nsec;
-        if (jp < 0) jp += nsec;
-        csv = D.Adiabatic ? cs[(size_t)i * nsec + j] : D.cs_ring[i];
-        Dn[i * nsec + j] = Dn[jp + (i - 1) * nsec];
-        En[i * nsec + j] = En[jp + (i - 1) * nsec];
-        Vrad_med = csv * (Dn[(i - 1) * nsec + j] - SigmaMed2) / SigmaMed2;
-        Vr[i * nsec + j] = 2. * Vrad_med - Vr[(i - 1) * nsec + j];
-      }
-      __syncthreads();
-      const size_t lo = (size_t)(nrad - 1) * nsec;
-      const float mean_dens_r = ref_device_reduce([&](long j) { return Dn[j]; }, nsec, sm) / (float)nsec;
-      const float mean_dens_r2 = ref_device_reduce([&](long j) { return Dn[lo + j]; }, nsec, sm) / (float)nsec;
-      const float mean_energy_r = ref_device_reduce([&](long j) { return En[j]; }, nsec, sm) / (float)nsec;
-      const float mean_energy_r2 = ref_device_reduce([&](long j) { return En[lo + j]; }, nsec, sm) / (float)nsec;
-      const float sm0 = D.SigmaMed[0], sm1 = D.SigmaMed[nrad - 1];
-      const float em0 = D.EnergyMed[0], em1 = D.EnergyMed[nrad - 1];
-      for (int j = tid; j < nsec; j += kThreads) {
-        Dn[j] += sm0 - mean_dens_r;
-        En[j] += em0 - mean_energy_r;
-        Dn[lo + j] += sm1 - mean_dens_r2;
-        En[lo + j] += em1 - mean_energy_r2;
-      }
-    }
+  const int ntile = na > 0 ? B.act_ring_off[na] : 0;
+  const int per = (ntile + gridDim.x - 1) / gridDim.x;
+  const int t0 = blockIdx.x * per, t1 = min(t0 + per, ntile);
+  int t = t0;
+  while (t < t1) {  // block-uniform: one disk per pass
+    const int a = find_range(B.act_ring_off, na, t);
+    const int lo = B.act_ring_off[a], te = min(t1, B.act_ring_off[a + 1]);
     __syncthreads();
+    copy_words(&sD, B.disks + B.act_disk[a], sizeof(DiskDev));
+    __syncthreads();
+    const DiskDev& D = sD;
+    DiskCtl* C = D.ctl;
+    const int nsec = D.nsec;
+    const int first = t, run = te - t;
+    t = te;
+    if (!D.IsDisk) continue;
+    const bool cs_rings = D.NonReflecting && D.Adiabatic;
+    const float dtf = C->dtf, domega = C->domega, OmegaFrame = C->OmegaFrame;
+    const float time_start = C->time_start, PTI = C->PhysicalTimeInitial;
+    for (int i = first - lo; (cs_rings || D.Evanescent) && i < te - lo; i++) {
+      const size_t r0 = (size_t)i * nsec;
+      if (cs_rings) {
+        float sum = 0.0f;  // Make1DprofileKernel: sectors in order
+        KahanSum ks;
+        const float gm = D.ADIABATICINDEX;
+        for (int c0 = 0; c0 < nsec; c0 += kBcCols) {
+          const int n = min(kBcCols, nsec - c0);
+          __syncthreads();
+#pragma unroll 4
+          for (int j = tid; j < n; j += kThreads) {
+            const float cs = sqrtf(gm * (gm - 1.0) * __ldg(D.energy + r0 + c0 + j) / __ldg(D.dens + r0 + c0 + j));
+            stg(D.cs + r0 + c0 + j, cs);
+            s_row[j] = cs;
+          }
+          __syncthreads();
+          if (tid == 0 && D.ViscosityAlpha) {
+            if (D.accurate) {
+              for (int j = 0; j < n; j++) ks.add(s_row[j]);
+            } else {
+              const float4* r4 = reinterpret_cast<const float4*>(s_row);
+              int j = 0;
+              for (; j + 32 <= n; j += 32) {
+                float4 v[8];
+#pragma unroll
+                for (int u = 0; u < 8; u++) v[u] = r4[(j >> 2) + u];
+#pragma unroll
+                for (int u = 0; u < 8; u++) {
+                  sum += v[u].x;
+                  sum += v[u].y;
+                  sum += v[u].z;
+                  sum += v[u].w;
+                }
+              }
+              for (; j < n; j++) sum += s_row[j];
+            }
+          }
+        }
+        if (tid == 0 && D.ViscosityAlpha) {
+          D.csmean[i] = (D.accurate ? ks.s : sum) / (float)nsec;
+          D.visc[i] = fviscosity_ring(D, i, time_start, PTI);
+        }
+      }
+      if (D.Evanescent) {
+        const float Rm = D.Rmed[i];
+        const bool corr = stage == 0 && domega != 0.0f;
+        const float DRMIN = D.ev_DRMIN, DRMAX = D.ev_DRMAX;
+        const bool damp = (Rm < DRMIN) || (Rm > DRMAX);
+        float lambda = 0.0f, vtheta0 = 0.0f, vrad0 = 0.0f;
+        if (damp) {
+          float damping;
+          if (Rm < DRMIN) {
+            damping = (Rm - DRMIN) / (D.Rmed[0] - DRMIN);
+            lambda = damping * damping * 10.0 * dtf / D.ev_Tin;
+          }
+          if (Rm > DRMAX) {
+            damping = (Rm - DRMAX) / (D.Rmed[D.nrad - 1] - DRMAX);
+            lambda = damping * damping * 10.0 * dtf / D.ev_Tout;
+          }
+          // the self-gravity form subtracts Rmed * GLOBAL_bufarray_d[i], an
+          // array the reference never fills (zero)
+          const float AspectRatio = aspect_ratio_dev(D, Rm, time_start, PTI);
+          vtheta0 = sqrtf(1.0 * 1.0 / Rm *
+                          (1.0 - (1.0 + D.SIGMASLOPE - 2.0 * D.FLARINGINDEX) * powf(AspectRatio, 2.0f) *
+                                     powf(Rm, (float)(2.0 * D.FLARINGINDEX))));
+          vtheta0 -= Rm * OmegaFrame;
+          vrad0 = -3.0 * D.visc[i] / Rm * (-D.SIGMASLOPE + .5);
+        } else if (!corr) {
+          continue;
+        }
+        const float dens0 = D.SigmaMed[i];
+        const float energy0 = D.EnergyMed[i];
+        const double den = 1.0 + lambda, rden = 1.0 / den;
+        const bool adi = D.Adiabatic;
+        float *pr = D.vrad + r0, *pt = D.vtheta + r0, *pd = D.dens + r0, *pe = D.energy + r0;
+        // the fields of four sectors are loaded before any is stored
+        for (int j0 = tid; j0 < nsec; j0 += 4 * kThreads) {
+          float vr[4], vt[4], dn[4], en[4];
+#pragma unroll
+          for (int u = 0; u < 4; u++) {
+            const int j = j0 + u * kThreads;
+            const bool ok = j < nsec;
+            vt[u] = ok ? pt[j] : 0.0f;
+            vr[u] = ok && damp ? pr[j] : 0.0f;
+            dn[u] = ok && damp ? pd[j] : 0.0f;
+            en[u] = ok && damp && adi ? pe[j] : 0.0f;
+          }
+#pragma unroll
+          for (int u = 0; u < 4; u++) {
+            const int j = j0 + u * kThreads;
+            if (j >= nsec) break;
+            if (corr) vt[u] = vt[u] - domega * Rm;
+            if (damp) {
+              vt[u] = div_by_recip_d(vt[u] + lambda * vtheta0, den, rden);
+              stg(pr + j, (float)div_by_recip_d(vr[u] + lambda * vrad0, den, rden));
+              stg(pd + j, (float)div_by_recip_d(dn[u] + lambda * dens0, den, rden));
+              if (adi) stg(pe + j, (float)div_by_recip_d(en[u] + lambda * energy0, den, rden));
+            }
+            stg(pt + j, vt[u]);
+          }
+        }
+      }
+    }
+    if (!(D.OpenInner || D.NonReflecting)) continue;
+    // the edge rings: after every ring's sound speed where there is one (the
+    // disk's ticket), else at once by the block of ring 0
+    if (cs_rings) {
+      __threadfence();
+      __syncthreads();
+      if (tid == 0) s_ticket = atomicAdd(&C->counter, (unsigned)run);
+      __syncthreads();
+      if (s_ticket + (unsigned)run != (unsigned)D.nrad) continue;
+      __threadfence();
+      if (tid == 0) C->counter = 0;
+    } else if (first != lo) {
+      continue;
+    }
+    boundary_edges(D, s_row);
   }
 }
 
@@ -3532,10 +3678,7 @@ void fargo_launch_substep(const BatchDev& b, cudaGraphConditionalHandle h, int u
   k_planets<<<b.ndisk, kThreads, 0, s>>>(b);
   if (fork) branch.leave();
   REC();
-  if (b.any_bc) {
-    k_bc_rings<0><<<b.ring_grid, kThreads, 0, s>>>(b);
-    k_bc_disk<<<b.ndisk, kThreads, 0, s>>>(b);
-  }
+  if (b.any_bc) k_boundary<0><<<b.ring_grid, kThreads, 0, s>>>(b);
   REC();
   if (b.src1_classes & 1) k_source1<0, 0><<<b.g_source1[0], kThreads, 0, s>>>(b);
   if (b.src1_classes & 2) k_source1<0, 1><<<b.g_source1[1], kThreads, 0, s>>>(b);
@@ -3547,10 +3690,7 @@ void fargo_launch_substep(const BatchDev& b, cudaGraphConditionalHandle h, int u
   if (b.ntheta_iso) k_source2<0><<<b.g_source2[0], kThreads, 0, s>>>(b);
   if (b.ntheta_adi) k_source2<1><<<b.g_source2[1], kThreads, 0, s>>>(b);
   REC();
-  if (b.any_bc) {
-    k_bc_rings<1><<<b.ring_grid, kThreads, 0, s>>>(b);
-    k_bc_disk<<<b.ndisk, kThreads, 0, s>>>(b);
-  }
+  if (b.any_bc) k_boundary<1><<<b.ring_grid, kThreads, 0, s>>>(b);
   REC();
   if (b.ntheta_adi) k_energy<<<b.g_energy, kThreads, 0, s>>>(b);  // adiabatic disks only
   REC();
@@ -3564,10 +3704,7 @@ void fargo_launch_substep(const BatchDev& b, cudaGraphConditionalHandle h, int u
   if (b.ntheta_iso) k_velocities<0><<<b.g_velocities[0], kThreads, 0, s>>>(b);
   if (b.ntheta_adi) k_velocities<1><<<b.g_velocities[1], kThreads, 0, s>>>(b);
   REC();
-  if (b.any_bc) {
-    k_bc_rings<2><<<b.ring_grid, kThreads, 0, s>>>(b);
-    k_bc_disk<<<b.ndisk, kThreads, 0, s>>>(b);
-  }
+  if (b.any_bc) k_boundary<2><<<b.ring_grid, kThreads, 0, s>>>(b);
   REC();
   if (fork) branch.join();
   k_substep_end<<<1, kThreads, 0, s>>>(b, h, use_handle);
@@ -3634,11 +3771,11 @@ cudaError_t fargo_size_grids(BatchDev& b, int nsm, long long ncell_tiles, int ni
 // Launches of one substep: 7 kernels, one Substep1 instance per kind of disk
 // present, the energy kernel when a disk is adiabatic, the isothermal and the
 // adiabatic forms of Substep2, transport and the velocity update when the
-// batch holds both, two per boundary call when a disk has a non-rigid
+// batch holds both, one per boundary call when a disk has a non-rigid
 // boundary.
 int fargo_substep_launches(const BatchDev& b) {
   return 7 + __builtin_popcount((unsigned)b.src1_classes) + (b.ntheta_adi ? 1 : 0) +
-         3 * ((b.ntheta_iso && b.ntheta_adi) ? 2 : 1) + (b.any_bc ? 6 : 0);
+         3 * ((b.ntheta_iso && b.ntheta_adi) ? 2 : 1) + (b.any_bc ? 3 : 0);
 }
 
 void fargo_launch_sector_tables(const BatchDev& b, int max_nsec, cudaStream_t s) {
