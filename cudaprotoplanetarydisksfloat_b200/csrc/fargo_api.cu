@@ -484,9 +484,14 @@ fargo_status build_graph(fargo_batch* b) {
   CK(cudaGraphAddNode(&node, b->graph, nullptr, 0, &cp));
   cudaGraph_t body = cp.conditional.phGraph_out[0];
   CK(cudaStreamBeginCaptureToGraph(b->stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
+  // the self-gravity beside the ring means, the CFL/force kernel and the potential
+  GraphBranch sg;
+  const bool fork = b->n_sg && sg.begin(b->stream);
   for (int d = 0; d < (int)b->disks.size(); d++)
     if (b->disks[d].sg) sg_capture_substep(b->disks[d].sg, b->bd, d, &b->disks[d].dev, b->stream);
-  fargo_launch_substep(b->bd, b->handle, 1, b->stream, b->max_nsec, nullptr);
+  if (fork) sg.leave();
+  fargo_launch_substep(b->bd, b->handle, 1, b->stream, b->max_nsec, nullptr, nullptr,
+                       FARGO_PART_HEAD | FARGO_PART_TAIL, fork ? &sg : nullptr);
   cudaError_t ec = cudaStreamEndCapture(b->stream, &body);
   if (ec != cudaSuccess) return set_err(b, FARGO_ECUDA, "graph capture: %s", cudaGetErrorString(ec));
   CK(cudaGraphInstantiate(&b->exec, b->graph, 0));

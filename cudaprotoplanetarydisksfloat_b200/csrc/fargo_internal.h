@@ -14,6 +14,7 @@
 //                 potential parameters, force sums, logs.
 #pragma once
 #include <cstdint>
+#include <vector>
 #include <cuda_runtime.h>
 
 #define FARGO_PI 3.14159265358979323844
@@ -202,6 +203,33 @@ struct BatchDev {
   int g_cfl, g_source1[4], g_potential, g_viscosity, g_source2[2], g_energy, g_velocities[2], g_transport;
 };
 
+// A side branch of a graph under capture, without a second stream: the nodes
+// launched between begin() and leave() become a branch, those after leave()
+// depend on what preceded begin(), and join() makes the next one depend on the
+// branch too.  begin() is false, and nothing happens, outside a capture.
+struct GraphBranch {
+  cudaStream_t s = nullptr;
+  std::vector<cudaGraphNode_t> before, tip;
+  static bool nodes(cudaStream_t s, std::vector<cudaGraphNode_t>& v) {
+    cudaStreamCaptureStatus st;
+    const cudaGraphNode_t* deps = nullptr;
+    size_t n = 0;
+    if (cudaStreamGetCaptureInfo(s, &st, nullptr, nullptr, &deps, &n) != cudaSuccess) return false;
+    if (st != cudaStreamCaptureStatusActive) return false;
+    v.assign(deps, deps + n);
+    return true;
+  }
+  bool begin(cudaStream_t stream) {
+    s = stream;
+    return nodes(s, before);
+  }
+  void leave() {
+    nodes(s, tip);
+    cudaStreamUpdateCaptureDependencies(s, before.data(), before.size(), cudaStreamSetCaptureDependencies);
+  }
+  void join() { cudaStreamUpdateCaptureDependencies(s, tip.data(), tip.size(), cudaStreamAddCaptureDependencies); }
+};
+
 // kernel entry points (kernels_step.cu), launched by fargo_api.cu
 #define FARGO_NKERNELS 15  // profiled slots per substep (boundary slots empty for rigid boundaries)
 #define FARGO_SEG_OUT 192  // largest azimuthal transport segment (output sectors per CTA)
@@ -217,6 +245,8 @@ struct BatchDev {
 #define FARGO_TR_ROWS_R (FARGO_BAND + 5)
 #define FARGO_TR_ROWS_T (FARGO_BAND + 4)
 // ev (optional): FARGO_NKERNELS+1 events, before each kernel and after the last.
+// sg (optional): the graph branch of the self-gravity, joined before the source
+// terms.
 // part: FARGO_PART_HEAD (ring means and CFL/forces), FARGO_PART_TAIL (the
 // rest: potential ... end of substep) or both.
 #define FARGO_PART_HEAD 1
@@ -237,7 +267,7 @@ struct BatchDev {
   void fargo_launch_cs_isothermal(const BatchDev& b, int only_disk, cudaStream_t s);                          \
   void fargo_launch_substep(const BatchDev& b, cudaGraphConditionalHandle h, int use_handle, cudaStream_t s,   \
                             int max_nsec, long long* launches, cudaEvent_t* ev = nullptr,                     \
-                            int part = FARGO_PART_HEAD | FARGO_PART_TAIL);                                     \
+                            int part = FARGO_PART_HEAD | FARGO_PART_TAIL, GraphBranch* sg = nullptr);           \
   /* radial stripes: the stripe's block for the gather (3 + 4 * bodies * own CFL tiles doubles), and the     \
      substep scalars from the gathered blocks (nonzero return: nstripe out of range) */                       \
   void fargo_launch_stripe_block(const BatchDev& b, double* out, cudaStream_t s);                             \

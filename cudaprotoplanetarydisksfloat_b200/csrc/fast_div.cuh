@@ -20,6 +20,13 @@ __device__ __forceinline__ float div_by_recip(float x, float d, float r) {
   return __fmaf_rn(e, r, q0);
 }
 
+// x / d in double from r = RN(1/d) (Markstein's method as in div_by_recip):
+// the correctly rounded quotient for normal operands, in three operations.
+__device__ __forceinline__ double div_by_recip_d(double x, double d, double r) {
+  const double q0 = __dmul_rn(x, r);
+  return __fma_rn(__fma_rn(-q0, d, x), r, q0);
+}
+
 // x / y for per-cell operands: the hardware's approximate reciprocal
 // (rcp.approx, relative error below 2^-22), then the same residual
 // correction: q0 = RN(x r), e = x - q0 y exact in one fused multiply-add,

@@ -46,7 +46,6 @@
 #include <algorithm>
 #include <cstdio>
 #include <type_traits>
-#include <vector>
 
 #include "fargo_internal.h"
 #include "fast_div.cuh"
@@ -3253,13 +3252,6 @@ __device__ void boundary_edges(const DiskDev& D, float* sm) {
   }
 }
 
-// x / d in double from r = RN(1/d) (Markstein's method as in div_by_recip):
-// the correctly rounded quotient for normal operands, in three operations.
-__device__ __forceinline__ double div_by_recip_d(double x, double d, double r) {
-  const double q0 = __dmul_rn(x, r);
-  return __fma_rn(__fma_rn(-q0, d, x), r, q0);
-}
-
 // ApplyBoundaryCondition (SideEuler.cu:172-182) of the disks inside their DT,
 // one launch: a block per ring (contiguous runs, DiskDev in shared memory), and
 // the edge rings by the block that completes a disk's last ring.
@@ -3613,35 +3605,8 @@ const char* fargo_substep_kernel_name(int k) {
   return (k >= 0 && k < FARGO_NKERNELS) ? names[k] : "";
 }
 
-// A side branch of a graph under capture, without a second stream: the nodes
-// launched between begin() and leave() become a branch, those after leave()
-// depend on what preceded begin(), and join() makes the next one depend on the
-// branch too.  begin() is false, and nothing happens, outside a capture.
-struct Branch {
-  cudaStream_t s = nullptr;
-  std::vector<cudaGraphNode_t> before, tip;
-  static bool nodes(cudaStream_t s, std::vector<cudaGraphNode_t>& v) {
-    cudaStreamCaptureStatus st;
-    const cudaGraphNode_t* deps = nullptr;
-    size_t n = 0;
-    if (cudaStreamGetCaptureInfo(s, &st, nullptr, nullptr, &deps, &n) != cudaSuccess) return false;
-    if (st != cudaStreamCaptureStatusActive) return false;
-    v.assign(deps, deps + n);
-    return true;
-  }
-  bool begin(cudaStream_t stream) {
-    s = stream;
-    return nodes(s, before);
-  }
-  void leave() {
-    nodes(s, tip);
-    cudaStreamUpdateCaptureDependencies(s, before.data(), before.size(), cudaStreamSetCaptureDependencies);
-  }
-  void join() { cudaStreamUpdateCaptureDependencies(s, tip.data(), tip.size(), cudaStreamAddCaptureDependencies); }
-};
-
 void fargo_launch_substep(const BatchDev& b, cudaGraphConditionalHandle h, int use_handle, cudaStream_t s,
-                          int max_nsec, long long* launches, cudaEvent_t* ev, int part) {
+                          int max_nsec, long long* launches, cudaEvent_t* ev, int part, GraphBranch* sg) {
   (void)max_nsec;
   int k = 0;
 #define REC()                                  \
@@ -3673,11 +3638,12 @@ void fargo_launch_substep(const BatchDev& b, cudaGraphConditionalHandle h, int u
   REC();
   // inside a graph the planets run beside the rest of the substep, unless its
   // kernels read the new frame
-  Branch branch;
+  GraphBranch branch;
   const bool fork = !b.any_corot && branch.begin(s);
   k_planets<<<b.ndisk, kThreads, 0, s>>>(b);
   if (fork) branch.leave();
   REC();
+  if (sg) sg->join();  // the source terms read the accelerations
   if (b.any_bc) k_boundary<0><<<b.ring_grid, kThreads, 0, s>>>(b);
   REC();
   if (b.src1_classes & 1) k_source1<0, 0><<<b.g_source1[0], kThreads, 0, s>>>(b);

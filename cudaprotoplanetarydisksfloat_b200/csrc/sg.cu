@@ -24,6 +24,7 @@
 #include <cstdio>
 #include <vector>
 
+#include "fast_div.cuh"
 #include "sg.h"
 
 #define PI_D FARGO_PI
@@ -43,20 +44,56 @@ struct SelfGravity {
 
 namespace {
 
+// The element-wise kernels take a run of a ring per thread: with V = 4 (NSEC a
+// multiple of 4) 16-byte words, else single cells; the ring's constants once.
+// Their divisions by constants of the disk are the IEEE quotients from the
+// constants' correctly rounded reciprocals (fast_div.cuh).
+template <int V>
+__device__ __forceinline__ bool sg_cell(const DiskDev& D, int& i, int& j) {
+  const long long c = V * ((long long)blockIdx.x * blockDim.x + threadIdx.x);
+  if (c >= (long long)D.nrad * D.nsec) return false;
+  i = (int)(c / D.nsec);
+  j = (int)(c - (long long)i * D.nsec);
+  return true;
+}
+template <int V>
+__device__ __forceinline__ void ld_run(float (&v)[V], const float* p) {
+  if constexpr (V == 4) {
+    const float4 t = __ldg(reinterpret_cast<const float4*>(p));
+    v[0] = t.x, v[1] = t.y, v[2] = t.z, v[3] = t.w;
+  } else {
+    v[0] = __ldg(p);
+  }
+}
+template <int V>
+__device__ __forceinline__ void st_run(float* p, const float (&v)[V]) {
+  if constexpr (V == 4)
+    *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+  else
+    p[0] = v[0];
+}
+
 // ComputeFFTKernel's density part (Kernels.cu:957-976) as real arrays, on
 // the rows that hold the density (the padding rows are the zero rows of the
 // row-spectrum buffer).
+template <int V>
 __global__ void k_sg_pad(DiskDev D, float* real2) {
-  const int nrad = D.nrad, nsec = D.nsec;
-  long long n = (long long)nrad * nsec;
-  long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= n) return;
-  if (!D.ctl->active) return;
-  int i = (int)(c / nsec), j = (int)(c - (long long)i * nsec);
-  float var = D.dens[c] * sqrtf(D.Rmed[i] / D.Rmed[0]);
+  int i, j;
+  if (!sg_cell<V>(D, i, j) || !D.ctl->active) return;
+  const int nsec = D.nsec;
+  const float R = D.Rmed[i], R0 = D.Rmed[0];
+  const float w = sqrtf(R / R0), r0 = 1.0f / R0;
+  float d[V], sr[V], st[V];
+  ld_run<V>(d, D.dens + (long long)i * nsec + j);
+#pragma unroll
+  for (int u = 0; u < V; u++) {
+    const float var = d[u] * w;
+    sr[u] = var;
+    st[u] = div_by_recip(var * R, R0, r0);
+  }
   float* row = real2 + 2LL * i * nsec + j;
-  row[0] = var;
-  row[nsec] = var * D.Rmed[i] / D.Rmed[0];
+  st_run<V>(row, sr);
+  st_run<V>(row + nsec, st);
 }
 
 // ComputeConvolutionKernel, Kernels.cu:980-999 (half spectrum): G = -K S
@@ -73,38 +110,75 @@ __global__ void k_sg_mul(const DiskCtl* C, float2* spec2, const float2* khat, lo
 }
 
 // ComputeSgAccKernel, Kernels.cu:1002-1021 (the C2R output is unnormalised,
-// as cufftExecC2C INVERSE is in the reference).
+// as cufftExecC2C INVERSE is in the reference).  The local term's products and
+// quotient are the reference's FP64 operations one by one.
+template <int V>
 __global__ void k_sg_acc(DiskDev D, const float* real2, float rstep, float tstep, float eps) {
+  int i, j;
+  if (!sg_cell<V>(D, i, j) || !D.ctl->active) return;
   const int nrad = D.nrad, nsec = D.nsec;
-  long long n = (long long)nrad * nsec;
-  long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= n) return;
-  if (!D.ctl->active) return;
-  int i = (int)(c / nsec), j = (int)(c - (long long)i * nsec);
+  const long long c = (long long)i * nsec + j;
   const float* row = real2 + 2LL * i * nsec + j;  // Gr, then Gphi one row on
+  float gr[V], gt[V], d[V], ar[V], at[V];
+  ld_run<V>(gr, row);
+  ld_run<V>(gt, row + nsec);
+  ld_run<V>(d, D.dens + c);
   float normaccr, normacct, divRmed;
   divRmed = D.Rmed[i] / D.Rmed[0];
   normaccr = rstep * tstep / ((float)(2 * nrad) * (float)nsec);
   normacct = normaccr;
   normaccr /= sqrtf(divRmed);
   normacct /= (divRmed * sqrtf(divRmed));
-  D.sg_acct[c] = row[nsec] * normacct;
-  float a = row[0] * normaccr;
-  a += 1.0 * D.dens[c] * rstep * tstep / eps;
-  D.sg_accr[c] = a;
+  const double deps = eps, reps = 1.0 / deps;
+#pragma unroll
+  for (int u = 0; u < V; u++) {
+    at[u] = gt[u] * normacct;
+    const float a = __fmul_rn(gr[u], normaccr);
+    ar[u] = (float)((double)a + div_by_recip_d(__dmul_rn(__dmul_rn((double)d[u], (double)rstep), (double)tstep), deps,
+                                               reps));
+  }
+  st_run<V>(D.sg_acct + c, at);
+  st_run<V>(D.sg_accr + c, ar);
 }
 
-// Make1Dprofile(2) at rings 0 and NRAD-1 (SideEuler.cu:261-267 needs only these)
-__global__ void k_sg_axi_edges(DiskDev D) {
+// Make1Dprofile(2) at rings 0 and NRAD-1 (SideEuler.cu:261-267 needs only
+// these), one block per ring: the ring's FP32 sum in sector order, a chain of
+// NSEC additions by one thread, its operands staged in shared memory by the
+// block and read 32 ahead as 16-byte words (from global memory, one thread at a
+// time, it took 21 us at 1024 sectors and 151 us at 6144; 4 and 22 us now).
+constexpr int kAxiCols = 4096;  // sectors staged at a time
+__global__ void __launch_bounds__(256) k_sg_axi_edges(DiskDev D) {
+  __shared__ __align__(16) float s_row[kAxiCols];
   if (!D.ctl->active) return;
-  int t = threadIdx.x;
-  if (t > 1) return;
-  int i = (t == 0) ? 0 : D.nrad - 1;
-  const float* f = D.sg_accr + (size_t)i * D.nsec;
+  const int i = blockIdx.x == 0 ? 0 : D.nrad - 1, tid = threadIdx.x, nsec = D.nsec;
+  const float* f = D.sg_accr + (size_t)i * nsec;
   float s = 0.0f;
-  for (int j = 0; j < D.nsec; j++) s += f[j];
-  s /= (float)D.nsec;
-  if (t == 0)
+  for (int c0 = 0; c0 < nsec; c0 += kAxiCols) {
+    const int n = min(kAxiCols, nsec - c0);
+    __syncthreads();
+#pragma unroll 4
+    for (int j = tid; j < n; j += 256) s_row[j] = f[c0 + j];
+    __syncthreads();
+    if (tid) continue;
+    const float4* r4 = reinterpret_cast<const float4*>(s_row);
+    int j = 0;
+    for (; j + 32 <= n; j += 32) {
+      float4 v[8];
+#pragma unroll
+      for (int u = 0; u < 8; u++) v[u] = r4[(j >> 2) + u];
+#pragma unroll
+      for (int u = 0; u < 8; u++) {
+        s += v[u].x;
+        s += v[u].y;
+        s += v[u].z;
+        s += v[u].w;
+      }
+    }
+    for (; j < n; j++) s += s_row[j];
+  }
+  if (tid) return;
+  s /= (float)nsec;
+  if (blockIdx.x == 0)
     D.ctl->axisg_in = s;
   else
     D.ctl->axisg_out = s;
@@ -288,14 +362,21 @@ void sg_capture_substep(SelfGravity* sg, const BatchDev& b, int d, DiskDev* D, c
   cufftSetStream(sg->col, s);
   cufftComplex* rows = reinterpret_cast<cufftComplex*>(sg->rows2);
   cufftComplex* spec = reinterpret_cast<cufftComplex*>(sg->spec2);
-  k_sg_pad<<<blocks(nr), 256, 0, s>>>(*D, sg->real2);
+  const bool vec = (sg->nsec & 3) == 0;
+  if (vec)
+    k_sg_pad<4><<<blocks(nr / 4), 256, 0, s>>>(*D, sg->real2);
+  else
+    k_sg_pad<1><<<blocks(nr), 256, 0, s>>>(*D, sg->real2);
   cufftExecR2C(sg->rowf, sg->real2, rows);                    // rows 0 .. nrad-1 of both fields
   cufftExecC2C(sg->col, rows, spec, CUFFT_FORWARD);          // all 2 nrad rows
   k_sg_mul<<<blocks(2 * nh), 256, 0, s>>>(D->ctl, sg->spec2, sg->khat, 2 * nh);
   cufftExecC2C(sg->col, spec, spec, CUFFT_INVERSE);
   cufftExecC2R(sg->rowi, spec, sg->real2);                    // rows 0 .. nrad-1 of both fields
-  k_sg_acc<<<blocks(nr), 256, 0, s>>>(*D, sg->real2, sg->rstep, sg->tstep, sg->eps);
-  k_sg_axi_edges<<<1, 32, 0, s>>>(*D);
+  if (vec)
+    k_sg_acc<4><<<blocks(nr / 4), 256, 0, s>>>(*D, sg->real2, sg->rstep, sg->tstep, sg->eps);
+  else
+    k_sg_acc<1><<<blocks(nr), 256, 0, s>>>(*D, sg->real2, sg->rstep, sg->tstep, sg->eps);
+  k_sg_axi_edges<<<2, 256, 0, s>>>(*D);
 }
 
 fargo_status sg_accelerations(SelfGravity* sg, const BatchDev& b, int d, DiskDev* D, cudaStream_t s,
