@@ -314,7 +314,11 @@ fargo_status make_tensor_maps(fargo_batch* b, DiskHost& h, DiskDev& D) {
   CUtensorMap* dm = nullptr;
   fargo_status st = dalloc(b, h, &dm, 3);
   if (st) return st;
-  CK(cudaMemcpy(dm, m, sizeof(m), cudaMemcpyHostToDevice));
+  // behind the buffer's clearing, on its stream (which the default stream does
+  // not wait for): a clearing that came last would leave the transport's TMA
+  // loads with empty maps
+  CK(cudaMemcpyAsync(dm, m, sizeof(m), cudaMemcpyHostToDevice, b->stream));
+  CK(cudaStreamSynchronize(b->stream));
   D.tmap = dm;
   return FARGO_OK;
 }
