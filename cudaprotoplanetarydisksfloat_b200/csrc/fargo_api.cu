@@ -103,6 +103,14 @@ fargo_status set_err(fargo_batch* b, fargo_status st, const char* fmt, ...) {
     }                                                                                          \
   } while (0)
 
+// Host-to-device copy in the order of the batch's stream, waited for.  (The
+// stream does not synchronise with the default stream, and a plain cudaMemcpy
+// from pageable memory may return before its last bytes have landed.)
+cudaError_t put(fargo_batch* b, void* dst, const void* src, size_t bytes) {
+  cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, b->stream);
+  return e != cudaSuccess ? e : cudaStreamSynchronize(b->stream);
+}
+
 template <class T>
 fargo_status dalloc(fargo_batch* b, DiskHost& h, T** ptr, size_t count) {
   void* p = nullptr;
@@ -317,8 +325,7 @@ fargo_status make_tensor_maps(fargo_batch* b, DiskHost& h, DiskDev& D) {
   // behind the buffer's clearing, on its stream (which the default stream does
   // not wait for): a clearing that came last would leave the transport's TMA
   // loads with empty maps
-  CK(cudaMemcpyAsync(dm, m, sizeof(m), cudaMemcpyHostToDevice, b->stream));
-  CK(cudaStreamSynchronize(b->stream));
+  CK(put(b, dm, m, sizeof(m)));
   D.tmap = dm;
   return FARGO_OK;
 }
@@ -394,7 +401,7 @@ fargo_status init_disk_state(fargo_batch* b, int d, const float* dens, const flo
   D.HillRadius = pl.nb > 0 ? (float)(pl.x[0] * std::pow(pl.mass[0] / 3., 1. / 3.)) : 0.0f;  // Psys.cu:206
   fargo_status st;
   if ((st = put_ctl_header(b, d, c))) return st;
-  CK(cudaMemcpy(b->d_disks + d, &D, sizeof(DiskDev), cudaMemcpyHostToDevice));
+  CK(put(b, b->d_disks + d, &D, sizeof(DiskDev)));
   if (p->SelfGravity) {
     // compute_selfgravity(init) + Init_planetarysys_withSG (Main.cu:302-329);
     // a radial stripe takes the whole disk's convolution on the whole
@@ -560,12 +567,11 @@ fargo_status install_items(fargo_batch* b) {
   b->d_theta = nullptr;
   CK(cudaMalloc(&b->d_theta, sizeof(int4) * (theta_iso.size() + theta_adi.size() + 1)));
   if (!theta_iso.empty())
-    CK(cudaMemcpy(b->d_theta, theta_iso.data(), sizeof(int4) * theta_iso.size(), cudaMemcpyHostToDevice));
+    CK(put(b, b->d_theta, theta_iso.data(), sizeof(int4) * theta_iso.size()));
   if (!theta_adi.empty())
-    CK(cudaMemcpy(b->d_theta + theta_iso.size(), theta_adi.data(), sizeof(int4) * theta_adi.size(),
-                  cudaMemcpyHostToDevice));
+    CK(put(b, b->d_theta + theta_iso.size(), theta_adi.data(), sizeof(int4) * theta_adi.size()));
   for (int d = 0; d < (int)b->disks.size(); d++)
-    CK(cudaMemcpy(&b->d_disks[d].item0, &b->disks[d].dev.item0, 2 * sizeof(int), cudaMemcpyHostToDevice));
+    CK(put(b, &b->d_disks[d].item0, &b->disks[d].dev.item0, 2 * sizeof(int)));
   BatchDev& bd = b->bd;
   bd.theta_iso = b->d_theta;
   bd.theta_adi = b->d_theta + theta_iso.size();
@@ -962,7 +968,7 @@ fargo_status fargo_checkpoint_load(fargo_ctx* ctx, const void* buf, size_t bytes
   CK(cudaStreamSynchronize(b->stream));
   const char* in = static_cast<const char*>(buf) + sizeof(hd);
   for (auto& p : ckpt_parts(b, 0)) {
-    CK(cudaMemcpy(p.dev, in, p.bytes, cudaMemcpyHostToDevice));
+    CK(put(b, p.dev, in, p.bytes));
     in += p.bytes;
   }
   return FARGO_OK;
@@ -1410,7 +1416,7 @@ fargo_status fargo_batch_set_max_substeps(fargo_batch* b, int n) {
   CK(cudaStreamSynchronize(b->stream));
   for (int d = 0; d < (int)b->disks.size(); d++) {
     b->disks[d].dev.max_sub = n;
-    CK(cudaMemcpy(&b->d_disks[d].max_sub, &n, sizeof(int), cudaMemcpyHostToDevice));
+    CK(put(b, &b->d_disks[d].max_sub, &n, sizeof(int)));
   }
   return FARGO_OK;
 }
@@ -1423,7 +1429,7 @@ fargo_status fargo_batch_set_precision(fargo_batch* b, int mode) {
   for (int d = 0; d < (int)b->disks.size(); d++) {
     DiskHost& h = b->disks[d];
     h.dev.accurate = acc;
-    CK(cudaMemcpy(&b->d_disks[d].accurate, &acc, sizeof(int), cudaMemcpyHostToDevice));
+    CK(put(b, &b->d_disks[d].accurate, &acc, sizeof(int)));
     if (h.sg) {
       fargo_status st = sg_tabulate(h.sg, h.t, acc, b->stream, b->err);
       if (st) return st;
@@ -1513,7 +1519,7 @@ fargo_status fargo_stripe_create(const fargo_params* p, const fargo_planets* pla
   b->ghost_lo = ring_lo - base;
   b->ghost_hi = top - ring_hi;
   set_cfl_tiles(b, (long long)NRAD * p->NSEC, b->device);  // the whole disk's tiles; sets bd.ncfl
-  CK(cudaMemcpy(b->d_disks, &D, sizeof(DiskDev), cudaMemcpyHostToDevice));
+  CK(put(b, b->d_disks, &D, sizeof(DiskDev)));
   if (p->SelfGravity) {
     // the whole disk's convolution: a view of the whole grid with its own
     // density buffer and ring tables, this stripe's control block
@@ -1529,7 +1535,7 @@ fargo_status fargo_stripe_create(const fargo_params* p, const fargo_planets* pla
     b->gallocs.push_back(gd);
     CK(cudaMalloc(&gr, sizeof(float) * (NRAD + 1)));
     b->gallocs.push_back(gr);
-    CK(cudaMemcpy(gr, b->gt.Rmed.data(), sizeof(float) * (NRAD + 1), cudaMemcpyHostToDevice));
+    CK(put(b, gr, b->gt.Rmed.data(), sizeof(float) * (NRAD + 1)));
     G.dens = gd;
     G.Rmed = gr;
     fargo_status sst = sg_create(&b->gsg, p, b->gt, b->stream, &G, b->err);
@@ -1558,7 +1564,7 @@ fargo_status fargo_stripe_init_state(fargo_ctx* ctx, const float* dens, const fl
         for (int j = 0; j < nsec; j++) S[(size_t)i * nsec + j] = b->gt.SigmaMed[i];
       src = S.data();
     }
-    CK(cudaMemcpy(b->gv.dens, src, sizeof(float) * (size_t)NRAD * nsec, cudaMemcpyHostToDevice));
+    CK(put(b, b->gv.dens, src, sizeof(float) * (size_t)NRAD * nsec));
   }
   return init_disk_state(b, 0, dens ? dens + off : nullptr, energy ? energy + off : nullptr);
 }
