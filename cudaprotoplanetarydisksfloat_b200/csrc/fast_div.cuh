@@ -35,13 +35,20 @@ __device__ __forceinline__ double div_by_recip_d(double x, double d, double r) {
 // boundary, and one ulp from it then (tests/test_gpu_division.py counts
 // both).  For normal y and quotient; four instructions against the IEEE
 // sequence's ~ten with its special-case branch.
-__device__ __forceinline__ float rcp_approx(float y) {
+//
+// The reciprocal is the flushing form: for a normal y (up to 2^125) it has the
+// bits of rcp.approx.f32, and its product with x those of __fdividef(x, y) (no
+// difference on 4e9 operand pairs), without the instructions by which those
+// handle a subnormal y; a subnormal y would count as zero.
+__device__ __forceinline__ float rcp_ftz(float y) {
   float r;
-  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(y));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(y));
   return r;
 }
+// the fast quotient (2 ulp) of normal operands
+__device__ __forceinline__ float div_fast(float x, float y) { return __fmul_rn(x, rcp_ftz(y)); }
 __device__ __forceinline__ float div_refined(float x, float y) {
-  const float r = rcp_approx(y);
+  const float r = rcp_ftz(y);
   const float q0 = __fmul_rn(x, r);
   return __fmaf_rn(__fmaf_rn(-q0, y, x), r, q0);
 }

@@ -1969,11 +1969,9 @@ __global__ void __launch_bounds__(kThreads, 3) k_energy(BatchDev B) {
 // ------------------------------------------------------------- transport
 
 // Transport arithmetic is FP32 throughout, and free of multiply-add
-// contraction: every product that meets an addition is an explicit
-// round-to-nearest multiply (fm), so each cell's result does not depend on
-// how the work is cut into bands, segments and unrolled steps (the compiler
-// may contract the same expression differently in different code paths).
-// The reference's own arithmetic, and the oracle's, is uncontracted too.
+// contraction by the compiler: every scalar product that meets an addition is
+// an explicit round-to-nearest multiply (fm), every paired addition says
+// whether it is fused (f2) or not (a2, s2).
 //
 // Transport arithmetic is FP32 throughout.  The reference writes several
 // of these expressions with double literals (0.5, 2.0, 1e-20), which
@@ -1990,32 +1988,39 @@ __global__ void __launch_bounds__(kThreads, 3) k_energy(BatchDev B) {
 // van Leer slope of StarRadKernel (Kernels.cu:917-927)
 __device__ __forceinline__ float fm(float a, float b) { return __fmul_rn(a, b); }
 
-// Paired FP32 arithmetic (Blackwell's two-lane FADD2 / FMUL2, round to
+// Paired FP32 arithmetic (Blackwell's two-lane FADD2 / FMUL2 / FFMA2, round to
 // nearest): a pair of quantities goes through one instruction, each lane
 // rounding as the scalar operation (no difference on 8.4 M operand pairs,
-// subnormals included).  Whole builds still differ in the last bits: the
-// paired azimuthal sweeps and the earlier scalar ones give fields ~5e-6
-// apart (rel-L2 of Sigma after 5 DTs), within the parity tolerances.
+// subnormals included).  The compiler may contract a paired product and the
+// addition that takes it into one fused operation, differently from one build
+// to the next, so the results would depend on code around them.  Here every
+// addition says which it is: f2 is the fused a*b + c; a2 and s2 are sums of
+// rounded operands, written as FFMA2 with the constants 1 and -1, which nothing
+// can be contracted into (and which cost what FADD2 costs).
 __device__ __forceinline__ float2 bc2(float x) { return make_float2(x, x); }
 __device__ __forceinline__ float2 m2(float2 a, float2 b) { return __fmul2_rn(a, b); }
-__device__ __forceinline__ float2 a2(float2 a, float2 b) { return __fadd2_rn(a, b); }
-__device__ __forceinline__ float2 s2(float2 a, float2 b) { return __fadd2_rn(a, make_float2(-b.x, -b.y)); }
+__device__ __forceinline__ float2 f2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+__device__ __forceinline__ float2 a2(float2 a, float2 b) { return __ffma2_rn(a, bc2(1.0f), b); }
+__device__ __forceinline__ float2 s2(float2 a, float2 b) { return __ffma2_rn(b, bc2(-1.0f), a); }
+// reciprocals of both lanes, see rcp_ftz
+__device__ __forceinline__ float2 rcp2(float2 a) { return make_float2(rcp_ftz(a.x), rcp_ftz(a.y)); }
 __device__ __forceinline__ float2 sel2(bool c, float2 a, float2 b) { return c ? a : b; }
 
 __device__ __forceinline__ float vl_rad_slope(float qm, float q0, float qp, float invdm, float invdp) {
   float dqm = fm(q0 - qm, invdm);
   float dqp = fm(qp - q0, invdp);
-  if (fm(dqp, dqm) > 0.0f) return __fdividef(fm(fm(2.0f, dqp), dqm), dqp + dqm);
-  return 0.0f;
+  const float g = div_fast(fm(fm(2.0f, dqp), dqm), dqp + dqm);
+  return fm(dqp, dqm) > 0.0f ? g : 0.0f;
 }
-// the same for two quantities at once
-__device__ __forceinline__ float2 vl_rad_slope2(float2 qm, float2 q0, float2 qp, float invdm, float invdp) {
-  const float2 dqm = m2(s2(q0, qm), bc2(invdm));
-  const float2 dqp = m2(s2(qp, q0), bc2(invdp));
+// the same for two quantities at once, from the differences q0 - qm and qp - q0
+__device__ __forceinline__ float2 vl_rad_slope2(float2 dm, float2 dp, float invdm, float invdp) {
+  const float2 dqm = m2(dm, bc2(invdm));
+  const float2 dqp = m2(dp, bc2(invdp));
   const float2 t = m2(dqp, dqm);
   const float2 num = m2(m2(bc2(2.0f), dqp), dqm);
   const float2 den = a2(dqp, dqm);
-  return make_float2(t.x > 0.0f ? __fdividef(num.x, den.x) : 0.0f, t.y > 0.0f ? __fdividef(num.y, den.y) : 0.0f);
+  const float2 g = m2(num, rcp2(den));
+  return make_float2(t.x > 0.0f ? g.x : 0.0f, t.y > 0.0f ? g.y : 0.0f);
 }
 
 // One row sample of the radial half of Transport at column g: the
@@ -2030,6 +2035,7 @@ struct RadRow {
   float S;         // density
   float2 Q[np];    // quantities, quantity nq-1 = S
   float2 W[np];    // quotients Q / (S + 1e-20)
+  float rden;      // 1 / (S + 1e-20)
 };
 template <int nq>
 __device__ __forceinline__ float lane_of(const float2 (&v)[(nq + 1) / 2], int c) {
@@ -2047,7 +2053,9 @@ struct TrView {
 
 // van Leer slopes at row r from rows r-1, r, r+1 (StarRadKernel; zero on the
 // first and last ring): g[] for the quotients, gs for the density.
-template <int nq>
+// fused: row r+1's density quotient enters its difference unrounded, Q rden - W
+// in one operation (see rad_march_s).
+template <int nq, bool fused = false>
 __device__ __forceinline__ void rad_slopes(const TrView& V, int r, const RadRow<nq>& A, const RadRow<nq>& Bm,
                                            const RadRow<nq>& Cp, float2* g, float& gs) {
   constexpr int np = RadRow<nq>::np;
@@ -2059,7 +2067,11 @@ __device__ __forceinline__ void rad_slopes(const TrView& V, int r, const RadRow<
   }
   const float im = __ldg(V.invdiffRmed + r), ip = __ldg(V.invdiffRmed + r + 1);
 #pragma unroll
-  for (int c = 0; c < np; c++) g[c] = vl_rad_slope2(A.W[c], Bm.W[c], Cp.W[c], im, ip);
+  for (int c = 0; c < np; c++) {
+    const float2 w = Bm.W[c];
+    const float2 dp = fused && c == np - 1 ? f2(Cp.Q[c], bc2(Cp.rden), make_float2(-w.x, -w.y)) : s2(Cp.W[c], w);
+    g[c] = vl_rad_slope2(s2(w, A.W[c]), dp, im, ip);
+  }
   gs = vl_rad_slope(A.S, Bm.S, Cp.S, im, ip);
 }
 
@@ -2086,7 +2098,7 @@ __device__ __forceinline__ void rad_face(const TrView& V, int b, float vr, float
   const float h = pos ? fm(rm - rl - fm(vr, dt), 0.5f) : fm(rp - rm + fm(vr, dt), 0.5f);
   const float hs = pos ? h : -h;
 #pragma unroll
-  for (int c = 0; c < np; c++) qs[c] = a2(sel2(pos, lo.W[c], hi.W[c]), m2(bc2(hs), sel2(pos, glo[c], ghi[c])));
+  for (int c = 0; c < np; c++) qs[c] = f2(bc2(hs), sel2(pos, glo[c], ghi[c]), sel2(pos, lo.W[c], hi.W[c]));
   ds = (pos ? lo.S : hi.S) + fm(hs, pos ? gslo : gshi);
 }
 
@@ -2124,7 +2136,8 @@ __device__ __forceinline__ RadRow<nq> rad_row_s(const TrView& V, const float* sI
     R.Q[2] = make_float2(__ldg(V.energy + rc * V.nsec + g), sg);
   else
     R.Q[2] = make_float2(sg, 0.0f);
-  const float rden = __fdividef(1.0f, sg + 1e-20f);
+  const float rden = rcp_ftz(sg + 1e-20f);
+  R.rden = rden;
 #pragma unroll
   for (int c = 0; c < np; c++) R.W[c] = m2(R.Q[c], bc2(rden));
   return R;
@@ -2162,7 +2175,14 @@ __device__ __forceinline__ void rad_march_s(const TrView& V, const float* sIn, i
     RadRow<nq> R3 = rad_row_s<nq>(V, sIn, i + 2, k + 4, p, g, Om);
     float2 G2[np], qs1[np];
     float gs2, ds1;
-    rad_slopes<nq>(V, i + 1, R1, R2, R3, G2, gs2);  // slope at row i+1
+    // slope at row i+1.  The isothermal form's last ring takes the outermost
+    // row's density quotient unrounded: no other expression needs it there, and
+    // the results of earlier builds, in which the compiler contracted just this
+    // product, stay what they were.
+    if (nq == 5 && k == FARGO_BAND - 1)
+      rad_slopes<nq, true>(V, i + 1, R1, R2, R3, G2, gs2);
+    else
+      rad_slopes<nq>(V, i + 1, R1, R2, R3, G2, gs2);
     const float vr1 = sIn[(kInR + k + 3) * kRow + p];  // row nrad is the zero ghost row
     rad_face<nq>(V, i + 1, vr1, dt, R1, R2, G1, gs1, G2, gs2, qs1, ds1);
     const float Ri = __ldg(V.Rinf + i), Rs = __ldg(V.Rsup + i), iS = __ldg(V.invSurf + i);
@@ -2171,9 +2191,9 @@ __device__ __forceinline__ void rad_march_s(const TrView& V, const float* sIn, i
     float2 varq[np];
 #pragma unroll
     for (int c = 0; c < np; c++) {
-      varq[c] = m2(m2(m2(bc2(fi), qs[c]), bc2(ds)), bc2(vr0));
-      varq[c] = s2(varq[c], m2(m2(m2(bc2(fs), qs1[c]), bc2(ds1)), bc2(vr1)));
-      const float2 r = a2(R1.Q[c], m2(varq[c], bc2(iS)));
+      const float2 out1 = m2(m2(m2(bc2(fs), qs1[c]), bc2(ds1)), bc2(vr1));
+      varq[c] = f2(m2(m2(bc2(fi), qs[c]), bc2(ds)), bc2(vr0), make_float2(-out1.x, -out1.y));
+      const float2 r = f2(varq[c], bc2(iS), R1.Q[c]);
       o[(2 * c) * ostride_c] = r.x;
       if (2 * c + 1 < nq) o[(2 * c + 1) * ostride_c] = r.y;
     }
@@ -2344,15 +2364,16 @@ __device__ __forceinline__ void sweep_pass(float* sRr, int b0, const float (&v)[
   auto slope = [&](float wm, float w0, float wp) -> float {
     float dqm = (w0 - wm);
     float dqp = (wp - w0);
-    if (fm(dqp, dqm) > 0.0f) return fm(__fdividef(fm(dqp, dqm), dqp + dqm), invdxtheta);
-    return 0.0f;
+    const float t = fm(dqp, dqm);
+    const float g = fm(div_fast(t, dqp + dqm), invdxtheta);
+    return t > 0.0f ? g : 0.0f;
   };
   auto slope2 = [&](float2 wm, float2 w0, float2 wp) -> float2 {
     const float2 dqm = s2(w0, wm);
     const float2 dqp = s2(wp, w0);
     const float2 t = m2(dqp, dqm);
     const float2 den = a2(dqp, dqm);
-    const float2 g = m2(make_float2(__fdividef(t.x, den.x), __fdividef(t.y, den.y)), bc2(invdxtheta));
+    const float2 g = m2(m2(t, rcp2(den)), bc2(invdxtheta));
     return make_float2(t.x > 0.0f ? g.x : 0.0f, t.y > 0.0f ? g.y : 0.0f);
   };
   auto shup2 = [](float2 x) -> float2 {
@@ -2371,7 +2392,7 @@ __device__ __forceinline__ void sweep_pass(float* sRr, int b0, const float (&v)[
   for (int k = 0; k < 8; k++) {
     vv[k] = (kind == 0) ? v[k] : vu;
     S[k] = sRr[(nq - 1) * kPad + b0 + k];
-    rr[k] = __fdividef(1.0f, S[k] + 1e-20f);
+    rr[k] = rcp_ftz(S[k] + 1e-20f);
     if (kind == 0) {
       const float ksi = fm(vv[k], dt);
       if (ksi > 0.0f) up |= 1u << k;
@@ -2413,7 +2434,7 @@ __device__ __forceinline__ void sweep_pass(float* sRr, int b0, const float (&v)[
       const bool u = is_left(k);
       const float2 xu = u ? (k ? X[k - 1] : Xl) : X[k];
       const float2 gu = u ? (k ? GX[k - 1] : GXl) : make_float2(-GX[k].x, -GX[k].y);
-      const float2 st = a2(xu, m2(bc2(h[k]), gu));  // (DensStar, the density's QRStar)
+      const float2 st = f2(bc2(h[k]), gu, xu);  // (DensStar, the density's QRStar)
       sD[k] = st.x;
       FX[k].x = fm(fm(fm(dxrad, st.y), st.x), vv[k]);  // the density's flux, left interface
     }
@@ -2446,7 +2467,7 @@ __device__ __forceinline__ void sweep_pass(float* sRr, int b0, const float (&v)[
       const bool u = is_left(k);
       const float2 wu = u ? (k ? W[k - 1] : Wl) : W[k];
       const float2 gu = u ? (k ? G[k - 1] : Gl) : make_float2(-G[k].x, -G[k].y);
-      const float2 qr = a2(wu, m2(bc2(h[k]), gu));
+      const float2 qr = f2(bc2(h[k]), gu, wu);
       F[k] = m2(m2(m2(bc2(dxrad), qr), bc2(sD[k])), bc2(vv[k]));  // flux through the left interface
     }
     const float2 Fr = shdn2(F[0]);
@@ -2454,7 +2475,7 @@ __device__ __forceinline__ void sweep_pass(float* sRr, int b0, const float (&v)[
 #pragma unroll
     for (int k = 0; k < 8; k++) {
       const float2 varq = s2(F[k], k < 7 ? F[k + 1] : Fr);
-      const float2 q = a2(make_float2(r0[k], r1[k]), m2(varq, bc2(invsurf)));  // unchanged rows: reread
+      const float2 q = f2(varq, bc2(invsurf), make_float2(r0[k], r1[k]));  // unchanged rows: reread
       r0[k] = q.x;
       r1[k] = q.y;
     }
@@ -2510,8 +2531,9 @@ __device__ __forceinline__ void sweep_pass(float (&q)[nq][8], const float (&v)[8
   auto slope = [&](float wm, float w0, float wp) -> float {
     float dqm = (w0 - wm);
     float dqp = (wp - w0);
-    if (fm(dqp, dqm) > 0.0f) return fm(__fdividef(fm(dqp, dqm), dqp + dqm), invdxtheta);
-    return 0.0f;
+    const float t = fm(dqp, dqm);
+    const float g = fm(div_fast(t, dqp + dqm), invdxtheta);
+    return t > 0.0f ? g : 0.0f;
   };
   // upwind side of each point's left interface and the distance to it:
   // ksi > 0 takes point k-1 at dxtheta - ksi, else point k at -(dxtheta + ksi)
@@ -2523,7 +2545,7 @@ __device__ __forceinline__ void sweep_pass(float (&q)[nq][8], const float (&v)[8
   for (int k = 0; k < 8; k++) {
     vv[k] = (kind == 0) ? v[k] : vu;
     S[k] = q[nq - 1][k];
-    rr[k] = __fdividef(1.0f, S[k] + 1e-20f);
+    rr[k] = rcp_ftz(S[k] + 1e-20f);
     if (kind == 0) {
       const float ksi = fm(vv[k], dt);
       if (ksi > 0.0f) up |= 1u << k;
