@@ -652,7 +652,8 @@ fargo_status batch_create(fargo_batch* b, int n, const fargo_params* params, con
   CK(cudaMalloc(&b->d_act_cell, sizeof(long long) * (n + 1)));
   CK(cudaMemsetAsync(b->d_act_cell, 0, sizeof(long long) * (n + 1), b->stream));
   b->red_blocks = 296;
-  CK(cudaMalloc(&b->d_red, sizeof(double) * b->red_blocks * 4 * FARGO_DIMFXY));
+  CK(cudaMalloc(&b->d_red, sizeof(double) * (FARGO_RED_HEAD + b->red_blocks * 4 * FARGO_DIMFXY)));
+  CK(cudaMemsetAsync(b->d_red, 0, sizeof(double) * FARGO_RED_HEAD, b->stream));
   CK(cudaMemcpyAsync(b->d_cell_off, cell_off.data(), sizeof(long long) * (n + 1), cudaMemcpyHostToDevice, b->stream));
   CK(cudaMemcpyAsync(b->d_ring_off, ring_off.data(), sizeof(int) * (n + 1), cudaMemcpyHostToDevice, b->stream));
   if (!theta_iso.empty())
@@ -1055,18 +1056,13 @@ static fargo_status disk_force_impl(fargo_batch* b, int d, double x, double y, d
   // ComputeForce (Force.cu:311-312): a and rh in double, kernel arguments float
   double a = std::sqrt(x * x + y * y);
   double rh = std::pow(mass / 3., 1. / 3.) * a + 1e-15;
+  const DiskDev& D = b->disks[d].dev;
   fargo_launch_disk_force(b->bd, d, (float)x, (float)y, (float)rsmoothing, (float)rh, (float)a, b->d_red,
-                          b->red_blocks, b->stream);
+                          fargo_red_blocks((long long)D.nrad * D.nsec, b->red_blocks), b->stream);
   CK(cudaGetLastError());
-  std::vector<double> part((size_t)b->red_blocks * 4 * FARGO_DIMFXY);
-  CK(cudaMemcpyAsync(part.data(), b->d_red, sizeof(double) * part.size(), cudaMemcpyDeviceToHost, b->stream));
+  CK(cudaMemcpyAsync(gf, b->d_red, sizeof(double) * 4 * FARGO_DIMFXY, cudaMemcpyDeviceToHost, b->stream));
   CK(cudaStreamSynchronize(b->stream));
   b->launches += 1;
-  for (int q = 0; q < 4 * FARGO_DIMFXY; q++) {
-    double s = 0;
-    for (int k = 0; k < b->red_blocks; k++) s += part[(size_t)k * 4 * FARGO_DIMFXY + q];
-    gf[q] = s;
-  }
   return FARGO_OK;
 }
 
@@ -1099,10 +1095,10 @@ static fargo_status scalars_impl(fargo_batch* b, int d, fargo_scalars* out) {
   cudaError_t e;
   DiskCtl c = ctl_header(b, d, &e);
   if (e != cudaSuccess) return set_err(b, FARGO_ECUDA, "%s", cudaGetErrorString(e));
-  fargo_launch_diagnostics(b->bd, d, b->d_red, b->red_blocks, b->stream);
+  fargo_launch_diagnostics(b->bd, d, b->d_red + FARGO_RED_HEAD, b->red_blocks, b->stream);
   CK(cudaGetLastError());
   std::vector<double> part((size_t)b->red_blocks * 3);
-  CK(cudaMemcpyAsync(part.data(), b->d_red, sizeof(double) * part.size(), cudaMemcpyDeviceToHost, b->stream));
+  CK(cudaMemcpyAsync(part.data(), b->d_red + FARGO_RED_HEAD, sizeof(double) * part.size(), cudaMemcpyDeviceToHost, b->stream));
   CK(cudaStreamSynchronize(b->stream));
   b->launches += 1;
   double m = 0, am = 0, hill = 0;

@@ -252,6 +252,13 @@ struct GraphBranch {
 #define FARGO_PART_HEAD 1
 #define FARGO_PART_TAIL 2
 #define FARGO_STRIPE_HEAD 3
+// The buffer of the disk-force sums: the results, a ticket (zero between
+// launches) in the last word of the head, then the blocks' partial sums.
+#define FARGO_RED_HEAD 64
+inline int fargo_red_blocks(long long cells, int most) {  // two cells a thread, at most `most` blocks
+  const long long n = (cells + 511) / 512;
+  return (int)(n < most ? n : most);
+}
 // The kernels and their launchers are compiled twice (kernels_step.cu):
 // fargo_k with the compiler's contraction of a*b+c into fused multiply-adds
 // (the reference-arithmetic precision mode, as the reference's own build)
@@ -276,7 +283,7 @@ struct GraphBranch {
   void fargo_launch_sector_tables(const BatchDev& b, int max_nsec, cudaStream_t s);                           \
   void fargo_launch_init_velocities(const BatchDev& b, int disk, long long ncell_ghost, cudaStream_t s);      \
   void fargo_launch_disk_force(const BatchDev& b, int disk, float x, float y, float rs, float rh, float a,     \
-                               double* out44, int nblocks, cudaStream_t s);                                   \
+                               double* red, int nblocks, cudaStream_t s);                                     \
   void fargo_launch_diagnostics(const BatchDev& b, int disk, double* out3, int nblocks, cudaStream_t s);      \
   int fargo_substep_launches(const BatchDev& b);                                                              \
   cudaError_t fargo_size_grids(BatchDev& b, int nsm, long long ncell_tiles, int nitems);                      \

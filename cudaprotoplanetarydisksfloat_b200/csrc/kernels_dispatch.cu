@@ -42,8 +42,8 @@ void fargo_launch_init_velocities(const BatchDev& b, int disk, long long ncell_g
   FARGO_BY_MODE(b, fargo_launch_init_velocities(b, disk, ncell_ghost, s));
 }
 void fargo_launch_disk_force(const BatchDev& b, int disk, float x, float y, float rs, float rh, float a,
-                             double* out44, int nblocks, cudaStream_t s) {
-  FARGO_BY_MODE(b, fargo_launch_disk_force(b, disk, x, y, rs, rh, a, out44, nblocks, s));
+                             double* red, int nblocks, cudaStream_t s) {
+  FARGO_BY_MODE(b, fargo_launch_disk_force(b, disk, x, y, rs, rh, a, red, nblocks, s));
 }
 void fargo_launch_diagnostics(const BatchDev& b, int disk, double* out3, int nblocks, cudaStream_t s) {
   FARGO_BY_MODE(b, fargo_launch_diagnostics(b, disk, out3, nblocks, s));
