@@ -21,7 +21,7 @@ NVFLAGS = ["-std=c++17", "-O3", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler"
            "-diag-suppress", "177", "-I" + os.path.join(ROOT, "include")]
 
 LIB_SOURCES = ["kernels_step.cu", "kernels_dispatch.cu", "fargo_api.cu", "sg.cu", "noalloc.cu", "host_params.cpp",
-               "host_setup.cpp"]
+               "host_setup.cpp", "host_copy.cpp"]
 # the step kernels a second time, without contraction of a*b+c into fused
 # multiply-adds: the accurate precision mode's kernel set
 VARIANTS = [("kernels_step.cu", "kernels_step_nofma.cu.o", ["-DFARGO_NOFMA", "-fmad=false"])]

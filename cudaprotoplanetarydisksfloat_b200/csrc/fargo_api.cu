@@ -22,6 +22,7 @@
 #include <vector>
 
 #include "fargo_internal.h"
+#include "host_copy.h"
 #include "host_internal.h"
 #include "sg.h"
 
@@ -47,6 +48,8 @@ struct fargo_batch {
   BatchDev bd{};
   DiskDev* d_disks = nullptr;
   DiskCtl* d_ctl = nullptr;
+  DiskCtl* h_ctl = nullptr;  // page-locked copy of the control blocks, and a few sums behind it
+  bool retained = false;     // a user of host_copy's rings
   long long* d_cell_off = nullptr;
   int* d_ring_off = nullptr;
   int4* d_theta = nullptr;
@@ -56,6 +59,7 @@ struct fargo_batch {
   long long* d_act_cell = nullptr;
   double* d_red = nullptr;  // reduction scratch for force/diagnostic kernels
   int red_blocks = 0;
+  static constexpr int kSums = 3 * 296 > 4 * FARGO_DIMFXY ? 3 * 296 : 4 * FARGO_DIMFXY;
   int max_nsec = 0;
   int any_adiabatic = 0;
   int n_sg = 0;
@@ -330,11 +334,14 @@ fargo_status make_tensor_maps(fargo_batch* b, DiskHost& h, DiskDev& D) {
   return FARGO_OK;
 }
 
+// The control block of a disk behind what the stream holds.
 DiskCtl ctl_header(const fargo_batch* b, int d, cudaError_t* e) {
-  DiskCtl c;
-  *e = cudaMemcpy(&c, b->d_ctl + d, sizeof(DiskCtl), cudaMemcpyDeviceToHost);
-  return c;
+  *e = cudaMemcpyAsync(b->h_ctl + d, b->d_ctl + d, sizeof(DiskCtl), cudaMemcpyDeviceToHost, b->stream);
+  if (*e == cudaSuccess) *e = cudaStreamSynchronize(b->stream);
+  return b->h_ctl[d];
 }
+// host room for the sums of the force and diagnostic calls
+double* host_sums(const fargo_batch* b) { return reinterpret_cast<double*>(b->h_ctl + b->disks.size()); }
 
 fargo_status put_ctl_header(fargo_batch* b, int d, const DiskCtl& c) {
   CK(cudaMemcpyAsync(b->d_ctl + d, &c, sizeof(DiskCtl), cudaMemcpyHostToDevice, b->stream));
@@ -641,6 +648,9 @@ fargo_status batch_create(fargo_batch* b, int n, const fargo_params* params, con
   seg_max = build_items(b, theta_iso, theta_adi);
   CK(cudaMalloc(&b->d_disks, sizeof(DiskDev) * n));
   CK(cudaMalloc(&b->d_ctl, sizeof(DiskCtl) * n));
+  CK(cudaMallocHost(&b->h_ctl, sizeof(DiskCtl) * n + sizeof(double) * b->kSums));
+  host_copy_retain();
+  b->retained = true;
   CK(cudaMemsetAsync(b->d_ctl, 0, sizeof(DiskCtl) * n, b->stream));
   CK(cudaMalloc(&b->d_cell_off, sizeof(long long) * (n + 1)));
   CK(cudaMalloc(&b->d_ring_off, sizeof(int) * (n + 1)));
@@ -736,6 +746,8 @@ void batch_free(fargo_batch* b) {
                 b->d_act, b->d_act_cell};
   for (void* p : ps)
     if (p) cudaFree(p);
+  if (b->h_ctl) cudaFreeHost(b->h_ctl);
+  if (b->retained) host_copy_release();
   if (b->stream) cudaStreamDestroy(b->stream);
 }
 
@@ -768,13 +780,14 @@ fargo_status advance_dt_async(fargo_batch* b) {
   return FARGO_OK;
 }
 
+// Waits for the stream and reports the disks' errors; the control blocks are
+// in h_ctl afterwards.
 fargo_status finish_dts(fargo_batch* b) {
+  CK(cudaMemcpyAsync(b->h_ctl, b->d_ctl, sizeof(DiskCtl) * b->disks.size(), cudaMemcpyDeviceToHost, b->stream));
   CK(cudaStreamSynchronize(b->stream));
   CK(cudaGetLastError());
   for (int d = 0; d < (int)b->disks.size(); d++) {
-    cudaError_t e;
-    DiskCtl c = ctl_header(b, d, &e);
-    if (e != cudaSuccess) return set_err(b, FARGO_ECUDA, "ctl read: %s", cudaGetErrorString(e));
+    const DiskCtl& c = b->h_ctl[d];
     if (c.error == 1) return set_err(b, FARGO_ENONFINITE, "disk %d: non-finite or non-positive CFL time step", d);
     if (c.error == 3)
       return set_err(b, FARGO_ETIMEOUT, "disk %d: a transport block gave up waiting for its staged rows", d);
@@ -865,25 +878,23 @@ static fargo_status download_impl(fargo_batch* b, int d, float* dens, float* vra
   size_t n = (size_t)(D.nrad + 1) * D.nsec;
   size_t bytes = sizeof(float) * n;
   std::vector<float> S, P, E;
-  if (dens) CK(cudaMemcpyAsync(dens, D.dens, bytes, cudaMemcpyDeviceToHost, b->stream));
-  if (vrad) CK(cudaMemcpyAsync(vrad, D.vrad, bytes, cudaMemcpyDeviceToHost, b->stream));
-  if (vtheta) CK(cudaMemcpyAsync(vtheta, D.vtheta, bytes, cudaMemcpyDeviceToHost, b->stream));
-  if (energy) CK(cudaMemcpyAsync(energy, D.energy, bytes, cudaMemcpyDeviceToHost, b->stream));
-  if (qplus) {
-    if (h.p.Adiabatic)
-      CK(cudaMemcpyAsync(qplus, D.qplus, bytes, cudaMemcpyDeviceToHost, b->stream));
-    else
-      std::memset(qplus, 0, bytes);
-  }
+  HostPiece piece[8];
+  int np = 0;
+  if (dens) piece[np++] = {dens, D.dens, bytes};
+  if (vrad) piece[np++] = {vrad, D.vrad, bytes};
+  if (vtheta) piece[np++] = {vtheta, D.vtheta, bytes};
+  if (energy) piece[np++] = {energy, D.energy, bytes};
+  if (qplus && h.p.Adiabatic) piece[np++] = {qplus, D.qplus, bytes};
+  if (qplus && !h.p.Adiabatic) std::memset(qplus, 0, bytes);
   if (temperature) {
     S.resize(n);
     P.resize(n);
     E.resize(n);
-    CK(cudaMemcpyAsync(S.data(), D.dens, bytes, cudaMemcpyDeviceToHost, b->stream));
-    CK(cudaMemcpyAsync(P.data(), D.pres, bytes, cudaMemcpyDeviceToHost, b->stream));
-    CK(cudaMemcpyAsync(E.data(), D.energy, bytes, cudaMemcpyDeviceToHost, b->stream));
+    piece[np++] = {S.data(), D.dens, bytes};
+    piece[np++] = {P.data(), D.pres, bytes};
+    piece[np++] = {E.data(), D.energy, bytes};
   }
-  CK(cudaStreamSynchronize(b->stream));
+  CK(host_copy(piece, np, b->device, b->stream));
   if (temperature) temperature_host(&h.p, S.data(), P.data(), E.data(), temperature, n, (size_t)D.nrad * D.nsec);
   return FARGO_OK;
 }
@@ -978,7 +989,6 @@ fargo_status fargo_checkpoint_load(fargo_ctx* ctx, const void* buf, size_t bytes
 static fargo_status get_planets_impl(fargo_batch* b, int d, fargo_planets* out) {
   if (!b || !out || d < 0 || d >= (int)b->disks.size()) return FARGO_EINVAL;
   CK(cudaSetDevice(b->device));
-  CK(cudaStreamSynchronize(b->stream));
   cudaError_t e;
   DiskCtl c = ctl_header(b, d, &e);
   if (e != cudaSuccess) return set_err(b, FARGO_ECUDA, "%s", cudaGetErrorString(e));
@@ -1022,11 +1032,7 @@ fargo_status fargo_advance_dt(fargo_ctx* ctx, int* nsub_out) {
   if (st) return st;
   st = finish_dts(b);
   if (st) return st;
-  if (nsub_out) {
-    cudaError_t e;
-    DiskCtl c = ctl_header(b, 0, &e);
-    *nsub_out = c.nsub;
-  }
+  if (nsub_out) *nsub_out = b->h_ctl[0].nsub;
   return FARGO_OK;
 }
 
@@ -1060,8 +1066,10 @@ static fargo_status disk_force_impl(fargo_batch* b, int d, double x, double y, d
   fargo_launch_disk_force(b->bd, d, (float)x, (float)y, (float)rsmoothing, (float)rh, (float)a, b->d_red,
                           fargo_red_blocks((long long)D.nrad * D.nsec, b->red_blocks), b->stream);
   CK(cudaGetLastError());
-  CK(cudaMemcpyAsync(gf, b->d_red, sizeof(double) * 4 * FARGO_DIMFXY, cudaMemcpyDeviceToHost, b->stream));
+  double* sums = host_sums(b);
+  CK(cudaMemcpyAsync(sums, b->d_red, sizeof(double) * 4 * FARGO_DIMFXY, cudaMemcpyDeviceToHost, b->stream));
   CK(cudaStreamSynchronize(b->stream));
+  std::memcpy(gf, sums, sizeof(double) * 4 * FARGO_DIMFXY);
   b->launches += 1;
   return FARGO_OK;
 }
@@ -1091,15 +1099,14 @@ fargo_status fargo_sg_accelerations(fargo_ctx* ctx, float* accr, float* acct) {
 static fargo_status scalars_impl(fargo_batch* b, int d, fargo_scalars* out) {
   if (!b || !out || d < 0 || d >= (int)b->disks.size()) return FARGO_EINVAL;
   CK(cudaSetDevice(b->device));
-  CK(cudaStreamSynchronize(b->stream));
-  cudaError_t e;
-  DiskCtl c = ctl_header(b, d, &e);
-  if (e != cudaSuccess) return set_err(b, FARGO_ECUDA, "%s", cudaGetErrorString(e));
   fargo_launch_diagnostics(b->bd, d, b->d_red + FARGO_RED_HEAD, b->red_blocks, b->stream);
   CK(cudaGetLastError());
-  std::vector<double> part((size_t)b->red_blocks * 3);
-  CK(cudaMemcpyAsync(part.data(), b->d_red + FARGO_RED_HEAD, sizeof(double) * part.size(), cudaMemcpyDeviceToHost, b->stream));
-  CK(cudaStreamSynchronize(b->stream));
+  double* part = host_sums(b);
+  CK(cudaMemcpyAsync(part, b->d_red + FARGO_RED_HEAD, sizeof(double) * 3 * b->red_blocks, cudaMemcpyDeviceToHost,
+                     b->stream));
+  cudaError_t e;
+  DiskCtl c = ctl_header(b, d, &e);  // waits for the sums too
+  if (e != cudaSuccess) return set_err(b, FARGO_ECUDA, "%s", cudaGetErrorString(e));
   b->launches += 1;
   double m = 0, am = 0, hill = 0;
   for (int k = 0; k < b->red_blocks; k++) {
