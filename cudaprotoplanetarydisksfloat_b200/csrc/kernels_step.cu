@@ -458,6 +458,22 @@ __device__ __forceinline__ void copy_words(void* dst, const void* src, int bytes
   for (int k = threadIdx.x; k < bytes / 4; k += blockDim.x) d[k] = s[k];
 }
 
+// Start of a chain kernel.  solo, an instance of its own: a batch of one disk
+// needs none of the lists of active disks (a substep runs only while the disk is
+// inside its DT), and its DiskDev, constant during a DT, is copied to shared
+// memory before the wait for the previous kernel, so that what is left after the
+// wait are the fields themselves, not a chain of four dependent loads (64x192:
+// 58.2 -> 56.0 us a substep, 256x768 adiabatic 72.7 -> 71.2; as a run-time choice in one
+// instance it cost the 16-disk sweep 1.5%).
+template <bool solo>
+__device__ __forceinline__ void chain_start(const BatchDev& B, DiskDev* sD) {
+  if (solo) {
+    copy_words(sD, B.disks, sizeof(DiskDev));
+    __syncthreads();
+  }
+  chain_wait();
+}
+
 // Four consecutive cells c0 .. c0+3 of one disk (c0 a multiple of 4).  With
 // vec (NSEC a multiple of 4) they share a ring, start at a sector multiple
 // of 4, and their fields load and store as 16-byte vectors; otherwise each
@@ -478,23 +494,25 @@ struct Quad {
 // -1: any): only the disks whose Adiabatic / SelfGravity flags match (the
 // energy kernel takes adiabatic disks, the Substep1 instances one kind each).
 static_assert(FARGO_QTILE == 4 * kThreads, "four cells per thread");
-template <int kAdi, int kSg, class Body>
+template <int kAdi, int kSg, bool solo, class Body>
 __device__ __forceinline__ void for_active_quads(const BatchDev& B, Body body) {
   __shared__ DiskDev sD;
-  if (B.ndisk == 1) copy_words(&sD, B.disks, sizeof(DiskDev));  // constant during a DT
-  chain_wait();
-  const int na = B.act[0];
+  chain_start<solo>(B, &sD);
+  const int na = solo ? 1 : B.act[0];
   if (na <= 0) return;
-  const int ntile = B.act_tile_off[na];
+  const int ntile = solo ? (int)(((long long)sD.nrad * sD.nsec + FARGO_QTILE - 1) / FARGO_QTILE) : B.act_tile_off[na];
   const int per = (ntile + gridDim.x - 1) / gridDim.x;
   const int t0 = blockIdx.x * per, t1 = min(t0 + per, ntile);
   int t = t0;
   while (t < t1) {  // block-uniform: one disk per pass
-    const int a = find_range(B.act_tile_off, na, t);
-    const int lo = B.act_tile_off[a], te = min(t1, B.act_tile_off[a + 1]);
-    __syncthreads();
-    if (B.ndisk > 1) copy_words(&sD, B.disks + B.act_disk[a], sizeof(DiskDev));
-    __syncthreads();
+    int lo = 0, te = t1;
+    if (!solo) {
+      const int a = find_range(B.act_tile_off, na, t);
+      lo = B.act_tile_off[a], te = min(t1, B.act_tile_off[a + 1]);
+      __syncthreads();
+      copy_words(&sD, B.disks + B.act_disk[a], sizeof(DiskDev));
+      __syncthreads();
+    }
     if (!sD.IsDisk || (kAdi >= 0 && (sD.Adiabatic != 0) != (kAdi == 1)) ||
         (kSg >= 0 && (sD.SelfGravity != 0) != (kSg == 1))) {  // nothing to do on this disk
       t = te;
@@ -625,7 +643,7 @@ __device__ __forceinline__ void qst(float* p, const Quad<V>& q, const float (&v)
 }
 
 #define QUAD_BEGIN_T(kAdi, kSg)                                                                         \
-  for_active_quads<kAdi, kSg>(B, [&](const DiskDev& D, const DiskCtl* C, const auto& q) {              \
+  for_active_quads<kAdi, kSg, solo>(B, [&](const DiskDev& D, const DiskCtl* C, const auto& q) {              \
     constexpr bool V = std::decay_t<decltype(q)>::vec;                                                 \
     (void)V;                                                                                           \
     const int nsec = D.nsec, nrad = D.nrad;                                                            \
@@ -1013,7 +1031,7 @@ static_assert(FARGO_CFL_TILE_SMALL == 4 * kThreads && FARGO_CFL_TILE % FARGO_CFL
 // double rounding innocuous for a quotient of two floats (Figueroa, "When is
 // double rounding innocuous?", SIGNUM 1995).
 static_assert(CFLSEC == 0.5, "the CFL limit's reciprocal form needs CFLSECURITY = 0.5");
-template <int NB>
+template <int NB, bool solo>
 __global__ void __launch_bounds__(kThreads, NB <= 1 ? 3 : 2) k_cfl_force(BatchDev B) {
   __shared__ DiskDev sD;
   __shared__ float s_b[5][NB];
@@ -1023,10 +1041,9 @@ __global__ void __launch_bounds__(kThreads, NB <= 1 ? 3 : 2) k_cfl_force(BatchDe
   __shared__ unsigned s_ticket;
   __shared__ int s_nbody;
   const int tid = threadIdx.x, w = tid >> 5, l = tid & 31;
-  if (B.ndisk == 1) copy_words(&sD, B.disks, sizeof(DiskDev));  // constant during a DT
-  chain_wait();
-  const int na = B.act[0];
-  const int ntile = na > 0 ? B.act_ctile_off[na] : 0;
+  chain_start<solo>(B, &sD);
+  const int na = solo ? 1 : B.act[0];
+  const int ntile = solo ? fargo_cfl_tiles_own(sD) : na > 0 ? B.act_ctile_off[na] : 0;
   const int per = (ntile + gridDim.x - 1) / gridDim.x;
   const int t0 = blockIdx.x * per, t1 = min(t0 + per, ntile);
   int lo = 0, hi = -1, run = 0;
@@ -1057,12 +1074,16 @@ __global__ void __launch_bounds__(kThreads, NB <= 1 ? 3 : 2) k_cfl_force(BatchDe
   for (int t = t0; t < t1; t++) {
     if (t >= hi) {  // block-uniform: entering a disk
       finish_run();
-      const int a = find_range(B.act_ctile_off, na, t);
-      lo = B.act_ctile_off[a];
-      hi = B.act_ctile_off[a + 1];
-      __syncthreads();
-      if (B.ndisk > 1) copy_words(&sD, B.disks + B.act_disk[a], sizeof(DiskDev));
-      __syncthreads();
+      if (solo) {
+        hi = ntile;
+      } else {
+        const int a = find_range(B.act_ctile_off, na, t);
+        lo = B.act_ctile_off[a];
+        hi = B.act_ctile_off[a + 1];
+        __syncthreads();
+        copy_words(&sD, B.disks + B.act_disk[a], sizeof(DiskDev));
+        __syncthreads();
+      }
       const DiskCtl* C = sD.ctl;
       const int nb = min(C->nbody, NB);
       if (tid == 0) s_nbody = nb;
@@ -1355,6 +1376,7 @@ __global__ void __launch_bounds__(kThreads) k_stripe_finish(BatchDev B, const do
 // per substep (Substep1 reads it at three cells each), summed over the
 // planets in the reference's order (FillForcesArraysKernel,
 // Kernels.cu:1322-1349); each planet's parameters are read once per quad.
+template <bool solo>
 __global__ void __launch_bounds__(kThreads) k_potential(BatchDev B) {
   QUAD_BEGIN
   float cp[4], sp[4], x[4], y[4], P[4];
@@ -1403,7 +1425,7 @@ __global__ void __launch_bounds__(kThreads) k_potential(BatchDev B) {
 // One instance per kind of disk (kAdi: adiabatic, kSg: self-gravity), so
 // that the isothermal form without self-gravity holds no energy or
 // acceleration samples and runs with more warps per SM.
-template <int kAdi, int kSg>
+template <int kAdi, int kSg, bool solo>
 __global__ void __launch_bounds__(kThreads, (kAdi == 0 && kSg == 0) ? 3 : 2) k_source1(BatchDev B) {
   QUAD_BEGIN_T(kAdi, kSg)
   const float dt = C->dtf;
@@ -1589,6 +1611,7 @@ __device__ __forceinline__ void cp_async_wait() {
 }
 
 constexpr size_t kViscSmem = sizeof(float) * 3 * 2 * kSR * kSC;  // dynamic: the staged tiles
+template <bool solo>
 __global__ void __launch_bounds__(kThreads, 3) k_viscosity(BatchDev B) {
   __shared__ DiskDev sD;
   extern __shared__ __align__(16) float vs_sm[];
@@ -1598,10 +1621,9 @@ __global__ void __launch_bounds__(kThreads, 3) k_viscosity(BatchDev B) {
   __shared__ float sD0b[2][kSR];
   __shared__ float sTrr[kTR][kTCp], sTpp[kTR][kTCp], sTrp[kTR][kTCp];
   const int tid = threadIdx.x;
-  if (B.ndisk == 1) copy_words(&sD, B.disks, sizeof(DiskDev));  // constant during a DT
-  chain_wait();
-  const int na = B.act[0];
-  const int ntile = na > 0 ? B.act_vtile_off[na] : 0;
+  chain_start<solo>(B, &sD);
+  const int na = solo ? 1 : B.act[0];
+  const int ntile = solo ? vtiles_of(sD) : na > 0 ? B.act_vtile_off[na] : 0;
   const int per = (ntile + gridDim.x - 1) / gridDim.x;
   const int t0 = blockIdx.x * per, t1 = min(t0 + per, ntile);
   // issue the asynchronous staging of tile lt of the disk in sD into buffer bf:
@@ -1651,12 +1673,16 @@ __global__ void __launch_bounds__(kThreads, 3) k_viscosity(BatchDev B) {
   bool have = false;  // tile t already staged (prefetched) in buffer bf
   for (int t = t0; t < t1; t++) {
     if (t >= hi) {  // block-uniform: entering a disk
-      const int a = find_range(B.act_vtile_off, na, t);
-      lo = B.act_vtile_off[a];
-      hi = B.act_vtile_off[a + 1];
-      __syncthreads();
-      if (B.ndisk > 1) copy_words(&sD, B.disks + B.act_disk[a], sizeof(DiskDev));
-      __syncthreads();
+      if (solo) {
+        hi = ntile;
+      } else {
+        const int a = find_range(B.act_vtile_off, na, t);
+        lo = B.act_vtile_off[a];
+        hi = B.act_vtile_off[a + 1];
+        __syncthreads();
+        copy_words(&sD, B.disks + B.act_disk[a], sizeof(DiskDev));
+        __syncthreads();
+      }
       have = false;
     }
     if (!have) stage(t - lo, bf);
@@ -1819,7 +1845,7 @@ __device__ __forceinline__ float qvisc(float dv, float dens) {
 
 // One instance per kind of disk (kAdi: adiabatic): the isothermal form holds
 // no energy samples.
-template <int kAdi>
+template <int kAdi, bool solo>
 __global__ void __launch_bounds__(kThreads, kAdi ? 3 : 4) k_source2(BatchDev B) {
   QUAD_BEGIN_T(kAdi, -1)
   const float dt = C->dtf;
@@ -1926,6 +1952,7 @@ __device__ __forceinline__ void qplus_quad(const DiskDev& D, const Quad<V>& q, i
   }
 }
 
+template <bool solo>
 __global__ void __launch_bounds__(kThreads, 3) k_energy(BatchDev B) {
   QUAD_BEGIN_T(1, -1)
   const float dt = C->dtf;
@@ -2254,17 +2281,18 @@ constexpr int kRMS = kRMW + 4;
 static_assert(kRMR <= 32 && kRMR * 4 <= 32, "one lane of warp 0 per ring, conflict-free 16-byte reads");
 static_assert(kRMW % 32 == 0 && kRMS % 4 == 0, "chunks of whole 32-sector blocks, 16-byte rows");
 size_t fargo_ring_mean_smem_bytes() { return sizeof(float) * 2 * kRMR * kRMS; }
-template <int mode>
+template <int mode, bool solo>
 __global__ void __launch_bounds__(kRMT) k_ring_mean(BatchDev B) {
   extern __shared__ __align__(16) float rm_sm[];  // [2][kRMR][kRMS]
-  chain_wait();
-  const int na = B.act[0];
-  const int ng = na > 0 ? B.act_grp_off[na] : 0;
+  __shared__ DiskDev sD;  // a batch of one disk
+  chain_start<solo>(B, &sD);
+  const int na = solo ? 1 : B.act[0];
+  const int ng = solo ? (sD.nrad + kRMR - 1) / kRMR : na > 0 ? B.act_grp_off[na] : 0;
   const int tid = threadIdx.x, lane = tid & 31;
   for (int g = blockIdx.x; g < ng; g += gridDim.x) {
-    const int a = find_range(B.act_grp_off, na, g);
-    const DiskDev& D = B.disks[B.act_disk[a]];
-    const int i0 = (g - B.act_grp_off[a]) * kRMR;
+    const int a = solo ? 0 : find_range(B.act_grp_off, na, g);
+    const DiskDev& D = solo ? sD : B.disks[B.act_disk[a]];
+    const int i0 = (solo ? g : g - B.act_grp_off[a]) * kRMR;
     const int nsec = D.nsec, nrad = D.nrad;
     const int nr = min(kRMR, nrad - i0);
     const float* base = D.vtheta + (size_t)i0 * nsec;
@@ -2700,7 +2728,8 @@ __device__ __forceinline__ void tma_load_2d(float* dst, const void* tmap, int x,
 }
 
 // Issue the asynchronous staging of transport item t's input rows (see
-// kRow).  With the disk's tensor maps (NSEC a multiple of 4, >= 64) one
+// kRow).  solo: the disk of a batch of one, in shared memory, else null.
+// With the disk's tensor maps (NSEC a multiple of 4, >= 64) one
 // thread issues three TMA box loads (Sigma, v_r, v_theta rows; rings outside
 // the disk come zero-filled) that complete on `bar`, and the call returns
 // true; columns of the window that wrap around the ring are then filled in
@@ -2710,14 +2739,13 @@ __device__ __forceinline__ void tma_load_2d(float* dst, const void* tmap, int x,
 // follow the azimuthal wrap themselves, and the call returns false.  The
 // choice depends only on the item and the disk: it is block-uniform.
 template <int nq>
-__device__ __forceinline__ bool tr_stage(const BatchDev& B, const int4* __restrict__ items, int t, float* sIn,
-                                         uint64_t* bar) {
-  const int nak = (nq == 5) ? B.act[1] : B.act[2];
+__device__ __forceinline__ bool tr_stage(const BatchDev& B, const DiskDev* solo, const int4* __restrict__ items, int t,
+                                         float* sIn, uint64_t* bar) {
   const int* aoff = (nq == 5) ? B.act_iso_off : B.act_adi_off;
   const int* adisk = (nq == 5) ? B.act_iso_disk : B.act_adi_disk;
-  const int a = find_range(aoff, nak, t);
-  const DiskDev& D = B.disks[adisk[a]];
-  const int4 it = items[D.item0 + (t - aoff[a])];
+  const int a = solo ? 0 : find_range(aoff, (nq == 5) ? B.act[1] : B.act[2], t);
+  const DiskDev& D = solo ? *solo : B.disks[adisk[a]];
+  const int4 it = items[D.item0 + (solo ? t : t - aoff[a])];
   const int i0 = it.y, g0 = it.z, W = it.w + 9;  // window + 1 columns
   const int nsec = D.nsec, nrad = D.nrad;
   if (D.tmap && (nsec & 3) == 0 && nsec >= 64 && (g0 & 3) == 0 && (smem_u32(sIn) & 127) == 0) {
@@ -2826,7 +2854,7 @@ __device__ __forceinline__ void tr_fixup(const DiskDev& D, int4 it, float* sIn) 
 // k_ring_mean<1>.  Final density / energy go to scratch (a0 / a1) because
 // neighbouring bands still read the old ones; the velocity kernel moves
 // them into the state.
-template <int nq>
+template <int nq, bool solo>
 __global__ void __launch_bounds__(kTT, 2) k_transport(BatchDev B, const int4* __restrict__ items) {
   extern __shared__ __align__(16) float tr_sm[];
   float* sR = tr_sm;                         // [kBR][nq + 1][kPad] radial results + v_theta
@@ -2837,26 +2865,27 @@ __global__ void __launch_bounds__(kTT, 2) k_transport(BatchDev B, const int4* __
   __shared__ float s_vmed[kBR], s_vc[kBR];
   __shared__ __align__(8) uint64_t s_bar;  // completion of the TMA staging
   __shared__ int s_gaveup;
-  chain_wait();
-  const int nak = (nq == 5) ? B.act[1] : B.act[2];
-  const int* aoff = (nq == 5) ? B.act_iso_off : B.act_adi_off;
-  const int* adisk = (nq == 5) ? B.act_iso_disk : B.act_adi_disk;
-  const int nai = nak > 0 ? aoff[nak] : 0;
+  __shared__ DiskDev sD;  // a batch of one disk
   const int p = threadIdx.x, warp = p >> 5, lane = p & 31;
   if (p == 0) {
     mbar_init(&s_bar, 1);
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     s_gaveup = 0;
   }
-  __syncthreads();
+  chain_start<solo>(B, &sD);
+  const int nak = solo ? 1 : (nq == 5) ? B.act[1] : B.act[2];
+  const int* aoff = (nq == 5) ? B.act_iso_off : B.act_adi_off;
+  const int* adisk = (nq == 5) ? B.act_iso_disk : B.act_adi_disk;
+  const int nai = solo ? sD.nitems : nak > 0 ? aoff[nak] : 0;
+  if (!solo) __syncthreads();
   unsigned phase = 0;  // parity of the staging barrier's next phase
   bool pend = false;   // a TMA staging is in flight
-  if ((int)blockIdx.x < nai) pend = tr_stage<nq>(B, items, blockIdx.x, sIn, &s_bar);
+  if ((int)blockIdx.x < nai) pend = tr_stage<nq>(B, solo ? &sD : nullptr, items, blockIdx.x, sIn, &s_bar);
   for (int t = blockIdx.x; t < nai; t += gridDim.x) {
     const int tn = t + gridDim.x;  // this block's next item
-    const int a = find_range(aoff, nak, t);
-    const DiskDev& D = B.disks[adisk[a]];
-    const int4 it = items[D.item0 + (t - aoff[a])];
+    const int a = solo ? 0 : find_range(aoff, nak, t);
+    const DiskDev& D = solo ? sD : B.disks[adisk[a]];
+    const int4 it = items[D.item0 + (solo ? t : t - aoff[a])];
     if (pend) {
       if (mbar_wait_bounded(&s_bar, phase)) {
         tr_fixup(D, it, sIn);
@@ -2876,7 +2905,7 @@ __global__ void __launch_bounds__(kTT, 2) k_transport(BatchDev B, const int4* __
     if (pend) phase ^= 1;
     pend = false;
     if (!D.IsDisk) {
-      if (tn < nai) pend = tr_stage<nq>(B, items, tn, sIn, &s_bar);
+      if (tn < nai) pend = tr_stage<nq>(B, solo ? &sD : nullptr, items, tn, sIn, &s_bar);
       continue;
     }
     const DiskCtl* C = D.ctl;
@@ -2905,7 +2934,7 @@ __global__ void __launch_bounds__(kTT, 2) k_transport(BatchDev B, const int4* __
       for (int r = 0; r < nb; r++) o[(r * (nq + 1) + nq) * kPad] = sIn[(kInT + r + 2) * kRow + p];
     }
     __syncthreads();  // radial results complete; the staged rows are free
-    if (tn < nai) pend = tr_stage<nq>(B, items, tn, sIn, &s_bar);
+    if (tn < nai) pend = tr_stage<nq>(B, solo ? &sD : nullptr, items, tn, sIn, &s_bar);
     const int r = warp;
     if (r < nb) {
       const int i = i0 + r;
@@ -2936,7 +2965,7 @@ __global__ void __launch_bounds__(kTT, 2) k_transport(BatchDev B, const int4* __
 // density (and energy, a1) become the state.
 // One instance per kind of disk (kAdi: adiabatic, which also moves the
 // transported energy into the state).
-template <int kAdi>
+template <int kAdi, bool solo>
 __global__ void __launch_bounds__(kThreads, kAdi ? 4 : 5) k_velocities(BatchDev B) {
   QUAD_BEGIN_T(kAdi, -1)
   const float Om = C->OmegaFrame;
@@ -3689,6 +3718,9 @@ const char* fargo_substep_kernel_name(int k) {
   return (k >= 0 && k < FARGO_NKERNELS) ? names[k] : "";
 }
 
+// The instance of a chain kernel for a batch of one disk (solo) or of several
+#define INST(k, ...) (solo ? k<__VA_ARGS__, true> : k<__VA_ARGS__, false>)
+
 // Launch in the chain: with pdl the kernel may start while the one before it in
 // the stream still runs (it waits for it itself, chain_wait).
 template <class... P, class... A>
@@ -3711,6 +3743,7 @@ void fargo_launch_substep(const BatchDev& b, cudaGraphConditionalHandle h, int u
   (void)max_nsec;
   // chained launches, unless each kernel is timed on its own
   const bool pdl = !ev;
+  const bool solo = b.ndisk == 1;
   int k = 0;
 #define REC()                                  \
   do {                                         \
@@ -3719,16 +3752,16 @@ void fargo_launch_substep(const BatchDev& b, cudaGraphConditionalHandle h, int u
   } while (0)
   if (part & FARGO_PART_HEAD) {
     REC();
-    go(k_ring_mean<0>, b.grp_grid, kRMT, fargo_ring_mean_smem_bytes(), s, false, b);
+    go(INST(k_ring_mean, 0), b.grp_grid, kRMT, fargo_ring_mean_smem_bytes(), s, false, b);
     REC();
     if (b.max_body <= 1)
-      go(k_cfl_force<1>, b.g_cfl, kThreads, 0, s, pdl, b);
+      go(INST(k_cfl_force, 1), b.g_cfl, kThreads, 0, s, pdl, b);
     else if (b.max_body <= 2)
-      go(k_cfl_force<2>, b.g_cfl, kThreads, 0, s, pdl, b);
+      go(INST(k_cfl_force, 2), b.g_cfl, kThreads, 0, s, pdl, b);
     else if (b.max_body <= 4)
-      go(k_cfl_force<4>, b.g_cfl, kThreads, 0, s, pdl, b);
+      go(INST(k_cfl_force, 4), b.g_cfl, kThreads, 0, s, pdl, b);
     else
-      go(k_cfl_force<FARGO_MAXBODY>, b.g_cfl, kThreads, 0, s, pdl, b);
+      go(INST(k_cfl_force, FARGO_MAXBODY), b.g_cfl, kThreads, 0, s, pdl, b);
   } else {
     k = 2;
   }
@@ -3737,7 +3770,7 @@ void fargo_launch_substep(const BatchDev& b, cudaGraphConditionalHandle h, int u
     return;
   }
   REC();
-  go(k_potential, b.g_potential, kThreads, 0, s, pdl && (part & FARGO_PART_HEAD), b);
+  go((solo ? k_potential<true> : k_potential<false>), b.g_potential, kThreads, 0, s, pdl && (part & FARGO_PART_HEAD), b);
   REC();
   // inside a graph the planets run beside the rest of the substep, unless its
   // kernels read the new frame
@@ -3750,31 +3783,35 @@ void fargo_launch_substep(const BatchDev& b, cudaGraphConditionalHandle h, int u
   bool chain = pdl && !sg;  // a kernel behind two branches waits for both in full
   if (b.any_bc) go(k_boundary<0>, b.ring_grid, kThreads, 0, s, std::exchange(chain, pdl), b);
   REC();
-  if (b.src1_classes & 1) go(k_source1<0, 0>, b.g_source1[0], kThreads, 0, s, std::exchange(chain, pdl), b);
-  if (b.src1_classes & 2) go(k_source1<0, 1>, b.g_source1[1], kThreads, 0, s, std::exchange(chain, pdl), b);
-  if (b.src1_classes & 4) go(k_source1<1, 0>, b.g_source1[2], kThreads, 0, s, std::exchange(chain, pdl), b);
-  if (b.src1_classes & 8) go(k_source1<1, 1>, b.g_source1[3], kThreads, 0, s, std::exchange(chain, pdl), b);
+  if (b.src1_classes & 1)
+    go(INST(k_source1, 0, 0), b.g_source1[0], kThreads, 0, s, std::exchange(chain, pdl), b);
+  if (b.src1_classes & 2)
+    go(INST(k_source1, 0, 1), b.g_source1[1], kThreads, 0, s, std::exchange(chain, pdl), b);
+  if (b.src1_classes & 4)
+    go(INST(k_source1, 1, 0), b.g_source1[2], kThreads, 0, s, std::exchange(chain, pdl), b);
+  if (b.src1_classes & 8)
+    go(INST(k_source1, 1, 1), b.g_source1[3], kThreads, 0, s, std::exchange(chain, pdl), b);
   REC();
-  go(k_viscosity, b.g_viscosity, kThreads, kViscSmem, s, pdl, b);
+  go((solo ? k_viscosity<true> : k_viscosity<false>), b.g_viscosity, kThreads, kViscSmem, s, pdl, b);
   REC();
-  if (b.ntheta_iso) go(k_source2<0>, b.g_source2[0], kThreads, 0, s, pdl, b);
-  if (b.ntheta_adi) go(k_source2<1>, b.g_source2[1], kThreads, 0, s, pdl, b);
+  if (b.ntheta_iso) go(INST(k_source2, 0), b.g_source2[0], kThreads, 0, s, pdl, b);
+  if (b.ntheta_adi) go(INST(k_source2, 1), b.g_source2[1], kThreads, 0, s, pdl, b);
   REC();
   if (b.any_bc) go(k_boundary<1>, b.ring_grid, kThreads, 0, s, pdl, b);
   REC();
-  if (b.ntheta_adi) go(k_energy, b.g_energy, kThreads, 0, s, pdl, b);  // adiabatic disks only
+  if (b.ntheta_adi) go((solo ? k_energy<true> : k_energy<false>), b.g_energy, kThreads, 0, s, pdl, b);  // adiabatic disks only
   REC();
-  go(k_ring_mean<1>, b.grp_grid, kRMT, fargo_ring_mean_smem_bytes(), s, pdl, b);
+  go(INST(k_ring_mean, 1), b.grp_grid, kRMT, fargo_ring_mean_smem_bytes(), s, pdl, b);
   REC();
   if (b.ntheta_iso)
-    go(k_transport<5>, std::min(b.g_transport, b.ntheta_iso), kTT, fargo_transport_smem_bytes(0), s, pdl, b,
+    go(INST(k_transport, 5), std::min(b.g_transport, b.ntheta_iso), kTT, fargo_transport_smem_bytes(0), s, pdl, b,
        b.theta_iso);
   if (b.ntheta_adi)
-    go(k_transport<6>, std::min(b.g_transport, b.ntheta_adi), kTT, fargo_transport_smem_bytes(1), s, pdl, b,
+    go(INST(k_transport, 6), std::min(b.g_transport, b.ntheta_adi), kTT, fargo_transport_smem_bytes(1), s, pdl, b,
        b.theta_adi);
   REC();
-  if (b.ntheta_iso) go(k_velocities<0>, b.g_velocities[0], kThreads, 0, s, pdl, b);
-  if (b.ntheta_adi) go(k_velocities<1>, b.g_velocities[1], kThreads, 0, s, pdl, b);
+  if (b.ntheta_iso) go(INST(k_velocities, 0), b.g_velocities[0], kThreads, 0, s, pdl, b);
+  if (b.ntheta_adi) go(INST(k_velocities, 1), b.g_velocities[1], kThreads, 0, s, pdl, b);
   REC();
   if (b.any_bc) go(k_boundary<2>, b.ring_grid, kThreads, 0, s, pdl, b);
   REC();
@@ -3798,18 +3835,21 @@ int fargo_launch_stripe_finish(const BatchDev& b, const double* blk, int nstripe
 // The transport kernels alone (both forms), for the autotuner: they read the
 // state and the last substep's ring means and write only scratch.
 void fargo_launch_transport(const BatchDev& b, cudaStream_t s) {
+  const bool solo = b.ndisk == 1;
   if (b.ntheta_iso)
-    k_transport<5><<<std::min(b.g_transport, b.ntheta_iso), kTT, fargo_transport_smem_bytes(0), s>>>(b, b.theta_iso);
+    go(INST(k_transport, 5), std::min(b.g_transport, b.ntheta_iso), kTT,
+       fargo_transport_smem_bytes(0), s, false, b, b.theta_iso);
   if (b.ntheta_adi)
-    k_transport<6><<<std::min(b.g_transport, b.ntheta_adi), kTT, fargo_transport_smem_bytes(1), s>>>(b, b.theta_adi);
+    go(INST(k_transport, 6), std::min(b.g_transport, b.ntheta_adi), kTT,
+       fargo_transport_smem_bytes(1), s, false, b, b.theta_adi);
 }
 
 // The CFL/force kernel instance for up to max_body bodies.
 const void* fargo_cfl_kernel(int max_body) {
-  return max_body <= 1   ? (const void*)k_cfl_force<1>
-         : max_body <= 2 ? (const void*)k_cfl_force<2>
-         : max_body <= 4 ? (const void*)k_cfl_force<4>
-                         : (const void*)k_cfl_force<FARGO_MAXBODY>;
+  return max_body <= 1   ? (const void*)k_cfl_force<1, false>
+         : max_body <= 2 ? (const void*)k_cfl_force<2, false>
+         : max_body <= 4 ? (const void*)k_cfl_force<4, false>
+                         : (const void*)k_cfl_force<FARGO_MAXBODY, false>;
 }
 
 // Grids of the substep kernels: one wave of resident blocks (the kernels walk
@@ -3826,18 +3866,18 @@ cudaError_t fargo_size_grids(BatchDev& b, int nsm, long long ncell_tiles, int ni
   };
   cudaError_t e;
   if ((e = wave(fargo_cfl_kernel(b.max_body), kThreads, 0, b.ncfl, &b.g_cfl))) return e;
-  if ((e = wave((const void*)k_source1<0, 0>, kThreads, 0, ncell_tiles, &b.g_source1[0]))) return e;
-  if ((e = wave((const void*)k_source1<0, 1>, kThreads, 0, ncell_tiles, &b.g_source1[1]))) return e;
-  if ((e = wave((const void*)k_source1<1, 0>, kThreads, 0, ncell_tiles, &b.g_source1[2]))) return e;
-  if ((e = wave((const void*)k_source1<1, 1>, kThreads, 0, ncell_tiles, &b.g_source1[3]))) return e;
-  if ((e = wave((const void*)k_potential, kThreads, 0, ncell_tiles, &b.g_potential))) return e;
-  if ((e = wave((const void*)k_viscosity, kThreads, kViscSmem, ncell_tiles, &b.g_viscosity))) return e;
-  if ((e = wave((const void*)k_source2<0>, kThreads, 0, ncell_tiles, &b.g_source2[0]))) return e;
-  if ((e = wave((const void*)k_source2<1>, kThreads, 0, ncell_tiles, &b.g_source2[1]))) return e;
-  if ((e = wave((const void*)k_energy, kThreads, 0, ncell_tiles, &b.g_energy))) return e;
-  if ((e = wave((const void*)k_velocities<0>, kThreads, 0, ncell_tiles, &b.g_velocities[0]))) return e;
-  if ((e = wave((const void*)k_velocities<1>, kThreads, 0, ncell_tiles, &b.g_velocities[1]))) return e;
-  return wave((const void*)k_transport<6>, kTT, fargo_transport_smem_bytes(1), nitems, &b.g_transport);
+  if ((e = wave((const void*)k_source1<0, 0, false>, kThreads, 0, ncell_tiles, &b.g_source1[0]))) return e;
+  if ((e = wave((const void*)k_source1<0, 1, false>, kThreads, 0, ncell_tiles, &b.g_source1[1]))) return e;
+  if ((e = wave((const void*)k_source1<1, 0, false>, kThreads, 0, ncell_tiles, &b.g_source1[2]))) return e;
+  if ((e = wave((const void*)k_source1<1, 1, false>, kThreads, 0, ncell_tiles, &b.g_source1[3]))) return e;
+  if ((e = wave((const void*)k_potential<false>, kThreads, 0, ncell_tiles, &b.g_potential))) return e;
+  if ((e = wave((const void*)k_viscosity<false>, kThreads, kViscSmem, ncell_tiles, &b.g_viscosity))) return e;
+  if ((e = wave((const void*)k_source2<0, false>, kThreads, 0, ncell_tiles, &b.g_source2[0]))) return e;
+  if ((e = wave((const void*)k_source2<1, false>, kThreads, 0, ncell_tiles, &b.g_source2[1]))) return e;
+  if ((e = wave((const void*)k_energy<false>, kThreads, 0, ncell_tiles, &b.g_energy))) return e;
+  if ((e = wave((const void*)k_velocities<0, false>, kThreads, 0, ncell_tiles, &b.g_velocities[0]))) return e;
+  if ((e = wave((const void*)k_velocities<1, false>, kThreads, 0, ncell_tiles, &b.g_velocities[1]))) return e;
+  return wave((const void*)k_transport<6, false>, kTT, fargo_transport_smem_bytes(1), nitems, &b.g_transport);
 }
 
 // Launches of one substep: 7 kernels, one Substep1 instance per kind of disk
@@ -3871,19 +3911,21 @@ void fargo_launch_diagnostics(const BatchDev& b, int disk, double* out3, int nbl
 
 cudaError_t fargo_kernel_attributes(int max_nsec) {
   (void)max_nsec;
-  cudaError_t e = cudaFuncSetAttribute(k_ring_mean<0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)fargo_ring_mean_smem_bytes());
-  if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(k_ring_mean<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)fargo_ring_mean_smem_bytes());
-  if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(k_viscosity, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kViscSmem);
-  if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(k_transport<5>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)fargo_transport_smem_bytes(0));
-  if (e != cudaSuccess) return e;
-  return cudaFuncSetAttribute(k_transport<6>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)fargo_transport_smem_bytes(1));
+  cudaError_t e = cudaSuccess;
+  auto smem = [&](const void* fn, size_t bytes) {
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  };
+  smem((const void*)k_ring_mean<0, false>, fargo_ring_mean_smem_bytes());
+  smem((const void*)k_ring_mean<0, true>, fargo_ring_mean_smem_bytes());
+  smem((const void*)k_ring_mean<1, false>, fargo_ring_mean_smem_bytes());
+  smem((const void*)k_ring_mean<1, true>, fargo_ring_mean_smem_bytes());
+  smem((const void*)k_viscosity<false>, kViscSmem);
+  smem((const void*)k_viscosity<true>, kViscSmem);
+  smem((const void*)k_transport<5, false>, fargo_transport_smem_bytes(0));
+  smem((const void*)k_transport<5, true>, fargo_transport_smem_bytes(0));
+  smem((const void*)k_transport<6, false>, fargo_transport_smem_bytes(1));
+  smem((const void*)k_transport<6, true>, fargo_transport_smem_bytes(1));
+  return e;
 }
 
 }  // namespace FARGO_KNS
