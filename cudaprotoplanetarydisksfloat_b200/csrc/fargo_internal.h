@@ -177,6 +177,7 @@ struct BatchDev {
   const int4* theta_adi;
   int ntheta_iso, ntheta_adi;
   int theta_seg;          // largest azimuthal segment (sectors)
+  int tr_narrow;          // the narrow transport (segments of at most FARGO_SEG_NARROW sectors)
   int* flags;             // [0] OR of the disks' "more" flags after a substep
   // compacted lists of the disks inside their DT (rebuilt on the device at the
   // start of a DT and after every substep): act[0] active disks, act[1] active
@@ -199,6 +200,7 @@ struct BatchDev {
   int accurate;              // precision mode of the batch's disks: which kernel set runs (FARGO_LAUNCHERS)
   int max_body;              // largest body count of the force sums (star + FeelDisk planets)
   // one-wave grids of the substep kernels (fargo_size_grids)
+  int ragged;                // some disk's NSEC is no multiple of 4
   int any_corot;             // some disk's frame corotates: its planets come before the source terms
   int g_cfl, g_source1[4], g_potential, g_viscosity, g_source2[2], g_energy, g_velocities[2], g_transport;
 };
@@ -235,6 +237,7 @@ struct GraphBranch {
 #define FARGO_SEG_OUT 192  // largest azimuthal transport segment (output sectors per CTA)
 #define FARGO_BAND 8       // rings per transport CTA
 #define FARGO_RM_RINGS 8   // rings per ring-mean CTA (serial FP32 chain per ring)
+#define FARGO_SEG_NARROW 120  // largest segment of the narrow transport (4 points a lane)
 #define FARGO_SEG_MAX 244  // widest segment the autotuner may pick: window + 1 = 253 <= FARGO_TR_ROW
 // Transport staging: each band's input rows are copied into shared memory as
 // rows of FARGO_TR_ROW columns (one TMA box of a 2-D tensor map per field):

@@ -2194,12 +2194,12 @@ __device__ __forceinline__ RadRow<nq> rad_row_s(const TrView& V, const float* sI
 // row, one new slope and one new interface.  out[k][c] at stride ostride.
 // lost0 (may be null): receives the density's varq at ring 0, the mass that
 // leaves through the inner edge (LostByDisk, Kernels.cu:941-944).
-// The rows come from the band's staged rows (ia = i0): window column p,
-// global column g.
-template <int nq>
+// The rows come from the band's staged rows, sIn and out at the band's ring of
+// ia: window column p, global column g.  NR: most rings; tail: they end the band.
+template <int nq, int NR>
 __device__ __forceinline__ void rad_march_s(const TrView& V, const float* sIn, int ia, int ib, int p, int g,
                                             float dt, float Om, float dtheta, float* out, int ostride_c,
-                                            int ostride_r, float* lost0) {
+                                            int ostride_r, float* lost0, bool tail) {
   constexpr int np = RadRow<nq>::np;
   RadRow<nq> R0 = rad_row_s<nq>(V, sIn, ia - 1, 1, p, g, Om);  // row i-1 for the first slope
   RadRow<nq> R1 = rad_row_s<nq>(V, sIn, ia, 2, p, g, Om);      // row i
@@ -2215,17 +2215,17 @@ __device__ __forceinline__ void rad_march_s(const TrView& V, const float* sIn, i
   rad_face<nq>(V, ia, vr0, dt, R0, R1, G0, gs0, G1, gs1, qs, ds);
   const float dtdth = fm(dt, dtheta);
 #pragma unroll
-  for (int k = 0; k < FARGO_BAND; k++) {
+  for (int k = 0; k < NR; k++) {
     const int i = ia + k;
     if (i >= ib) break;
     RadRow<nq> R3 = rad_row_s<nq>(V, sIn, i + 2, k + 4, p, g, Om);
     float2 G2[np], qs1[np];
     float gs2, ds1;
-    // slope at row i+1.  The isothermal form's last ring takes the outermost
+    // slope at row i+1.  The isothermal form's last ring of a band takes the outermost
     // row's density quotient unrounded: no other expression needs it there, and
     // the results of earlier builds, in which the compiler contracted just this
     // product, stay what they were.
-    if (nq == 5 && k == FARGO_BAND - 1)
+    if (nq == 5 && k == NR - 1 && tail)
       rad_slopes<nq, true>(V, i + 1, R1, R2, R3, G2, gs2);
     else
       rad_slopes<nq>(V, i + 1, R1, R2, R3, G2, gs2);
@@ -2380,20 +2380,31 @@ __global__ void __launch_bounds__(kRMT) k_ring_mean(BatchDev B) {
 
 constexpr int kTT = 256;         // threads of the transport kernel
 constexpr int kBR = FARGO_BAND;  // rings per transport band: one warp each in the sweeps
-constexpr int kPad = kTT + kTT / 8;  // shared row with a padding word after every 8
 static_assert(FARGO_SEG_OUT + 8 <= kTT, "transport window must fit the CTA");
 static_assert(kBR * 32 == kTT, "one warp per ring of the band");
 
-// padded shared-memory index: 8 consecutive points per lane read without
-// bank conflicts, 32 consecutive points per warp too
-__device__ __forceinline__ int pidx(int t) { return t + (t >> 3); }
+// A lane holds P consecutive points of its ring in the sweeps: 8 (windows of
+// 256 columns), or 4 (of 128) where the items are so few that the chip idles: a
+// block then takes half as long, its radial half runs as two half-bands side by
+// side, and there are twice as many (BatchDev::tr_narrow).
+// Padded shared-memory index: P consecutive points per lane read without
+// bank conflicts, 32 consecutive points per warp too (a padding word after every
+// P: lane strides 9 and 5).
+template <int P>
+constexpr int kPad = 32 * (P + 1);  // a shared row
+template <int P>
+__device__ __forceinline__ int pidx(int t) {
+  return t + t / P;
+}
 
-size_t fargo_transport_smem_bytes(int adiabatic) {
+template <int P>
+size_t transport_smem_bytes(int adiabatic) {
   const int nq = adiabatic ? 6 : 5;
   // + 128: the staged rows start on a 128-byte boundary
-  return sizeof(float) * ((size_t)kPad * (size_t)(kBR * (nq + 1) + 1) + (size_t)kInRows * kRow) + 128;
+  return sizeof(float) * ((size_t)kPad<P> * (size_t)(kBR * (nq + 1) + 1) + (size_t)kInRows * kRow) + 128;
 }
-static_assert((kPad * 4) % 16 == 0 && (kRow * 4) % 16 == 0, "staged rows 16-byte aligned");
+static_assert((kPad<8> * 4) % 16 == 0 && (kPad<4> * 4) % 16 == 0 && (kRow * 4) % 16 == 0, "staged rows aligned");
+static_assert(FARGO_SEG_NARROW + 8 <= 128 && (FARGO_SEG_NARROW & 3) == 0, "a narrow window fits 4 points a lane");
 
 #ifndef FARGO_NOFMA
 // One van Leer pass of OneWindTheta on the window (see sweep_ring).  kind 0:
@@ -2402,12 +2413,12 @@ static_assert((kPad * 4) % 16 == 0 && (kRow * 4) % 16 == 0, "staged rows 16-byte
 // interfaces all take their upwind value from the left (1: vu dt > 0) or
 // from the right (2), at the same distance h: no per-point selects.
 // The quantities stay in the ring's shared-memory rows (each lane reads and
-// writes only its own 8 points there); they are processed two at a time as
+// writes only its own points there); they are processed two at a time as
 // the lanes of paired FP32 operations (each lane rounds as the scalar
 // operation); with an odd count the last quantity, the density, shares a
 // pair with its own star value.
-template <int nq, int kind>
-__device__ __forceinline__ void sweep_pass(float* sRr, int b0, const float (&v)[8], float vu, float dt,
+template <int nq, int kind, int P>
+__device__ __forceinline__ void sweep_pass(float* sRr, int b0, const float (&v)[P], float vu, float dt,
                                            float dxtheta, float invdxtheta, float invsurf, float dxrad) {
   auto slope = [&](float wm, float w0, float wp) -> float {
     float dqm = (w0 - wm);
@@ -2432,14 +2443,14 @@ __device__ __forceinline__ void sweep_pass(float* sRr, int b0, const float (&v)[
   };
   // upwind side of each point's left interface and the distance to it:
   // ksi > 0 takes point k-1 at dxtheta - ksi, else point k at -(dxtheta + ksi)
-  float vv[8], rr[8], S[8], GS[8], sD[8], h[8];
+  float vv[P], rr[P], S[P], GS[P], sD[P], h[P];
   unsigned up = 0;
   const float ksu = fm(vu, dt);
   const float hu = (kind == 1) ? dxtheta - ksu : dxtheta + ksu;
 #pragma unroll
-  for (int k = 0; k < 8; k++) {
+  for (int k = 0; k < P; k++) {
     vv[k] = (kind == 0) ? v[k] : vu;
-    S[k] = sRr[(nq - 1) * kPad + b0 + k];
+    S[k] = sRr[(nq - 1) * kPad<P> + b0 + k];
     rr[k] = rcp_ftz(S[k] + 1e-20f);
     if (kind == 0) {
       const float ksi = fm(vv[k], dt);
@@ -2451,14 +2462,14 @@ __device__ __forceinline__ void sweep_pass(float* sRr, int b0, const float (&v)[
   }
   auto is_left = [&](int k) -> bool { return kind == 0 ? ((up >> k) & 1u) != 0 : kind == 1; };
   if constexpr ((nq & 1) == 0) {
-    const float Sl = __shfl_up_sync(0xffffffffu, S[7], 1);
+    const float Sl = __shfl_up_sync(0xffffffffu, S[P - 1], 1);
     const float Sr = __shfl_down_sync(0xffffffffu, S[0], 1);
 #pragma unroll
-    for (int k = 0; k < 8; k++) GS[k] = slope(k ? S[k - 1] : Sl, S[k], k < 7 ? S[k + 1] : Sr);
-    const float GSl = (kind == 2) ? 0.0f : __shfl_up_sync(0xffffffffu, GS[7], 1);
+    for (int k = 0; k < P; k++) GS[k] = slope(k ? S[k - 1] : Sl, S[k], k < P - 1 ? S[k + 1] : Sr);
+    const float GSl = (kind == 2) ? 0.0f : __shfl_up_sync(0xffffffffu, GS[P - 1], 1);
     // DensStar (StarThetaKernel2 on the density); a - fm(h, g) = a + fm(h, -g)
 #pragma unroll
-    for (int k = 0; k < 8; k++) {
+    for (int k = 0; k < P; k++) {
       const bool u = is_left(k);
       const float su = u ? (k ? S[k - 1] : Sl) : S[k];
       const float gu = u ? (k ? GS[k - 1] : GSl) : -GS[k];
@@ -2469,16 +2480,16 @@ __device__ __forceinline__ void sweep_pass(float* sRr, int b0, const float (&v)[
     // interface value are the same slope and upwind expressions, on Sigma and
     // on Sigma / (Sigma + 1e-20): the two lanes of one pair.  The density row
     // is updated at once (the pairs below read only their own rows).
-    float2 X[8], GX[8], FX[8];
+    float2 X[P], GX[P], FX[P];
 #pragma unroll
-    for (int k = 0; k < 8; k++) X[k] = make_float2(S[k], fm(S[k], rr[k]));
-    const float2 Xl = shup2(X[7]);
+    for (int k = 0; k < P; k++) X[k] = make_float2(S[k], fm(S[k], rr[k]));
+    const float2 Xl = shup2(X[P - 1]);
     const float2 Xr = shdn2(X[0]);
 #pragma unroll
-    for (int k = 0; k < 8; k++) GX[k] = slope2(k ? X[k - 1] : Xl, X[k], k < 7 ? X[k + 1] : Xr);
-    const float2 GXl = (kind == 2) ? bc2(0.0f) : shup2(GX[7]);
+    for (int k = 0; k < P; k++) GX[k] = slope2(k ? X[k - 1] : Xl, X[k], k < P - 1 ? X[k + 1] : Xr);
+    const float2 GXl = (kind == 2) ? bc2(0.0f) : shup2(GX[P - 1]);
 #pragma unroll
-    for (int k = 0; k < 8; k++) {
+    for (int k = 0; k < P; k++) {
       const bool u = is_left(k);
       const float2 xu = u ? (k ? X[k - 1] : Xl) : X[k];
       const float2 gu = u ? (k ? GX[k - 1] : GXl) : make_float2(-GX[k].x, -GX[k].y);
@@ -2487,11 +2498,11 @@ __device__ __forceinline__ void sweep_pass(float* sRr, int b0, const float (&v)[
       FX[k].x = fm(fm(fm(dxrad, st.y), st.x), vv[k]);  // the density's flux, left interface
     }
     const float Fr = __shfl_down_sync(0xffffffffu, FX[0].x, 1);
-    float* rd = sRr + (nq - 1) * kPad + b0;
+    float* rd = sRr + (nq - 1) * kPad<P> + b0;
 #pragma unroll
-    for (int k = 0; k < 8; k++) {
+    for (int k = 0; k < P; k++) {
       float varq = FX[k].x;
-      varq -= (k < 7 ? FX[k + 1].x : Fr);
+      varq -= (k < P - 1 ? FX[k + 1].x : Fr);
       rd[k] = S[k] + fm(varq, invsurf);
     }
   }
@@ -2500,18 +2511,18 @@ __device__ __forceinline__ void sweep_pass(float* sRr, int b0, const float (&v)[
   constexpr int npair = nq / 2;
 #pragma unroll
   for (int c2 = 0; c2 < npair; c2++) {
-    float* r0 = sRr + (2 * c2) * kPad + b0;
-    float* r1 = r0 + kPad;
-    float2 W[8], G[8], F[8];
+    float* r0 = sRr + (2 * c2) * kPad<P> + b0;
+    float* r1 = r0 + kPad<P>;
+    float2 W[P], G[P], F[P];
 #pragma unroll
-    for (int k = 0; k < 8; k++) W[k] = m2(make_float2(r0[k], r1[k]), bc2(rr[k]));
-    const float2 Wl = shup2(W[7]);
+    for (int k = 0; k < P; k++) W[k] = m2(make_float2(r0[k], r1[k]), bc2(rr[k]));
+    const float2 Wl = shup2(W[P - 1]);
     const float2 Wr = shdn2(W[0]);
 #pragma unroll
-    for (int k = 0; k < 8; k++) G[k] = slope2(k ? W[k - 1] : Wl, W[k], k < 7 ? W[k + 1] : Wr);
-    const float2 Gl = (kind == 2) ? bc2(0.0f) : shup2(G[7]);
+    for (int k = 0; k < P; k++) G[k] = slope2(k ? W[k - 1] : Wl, W[k], k < P - 1 ? W[k + 1] : Wr);
+    const float2 Gl = (kind == 2) ? bc2(0.0f) : shup2(G[P - 1]);
 #pragma unroll
-    for (int k = 0; k < 8; k++) {
+    for (int k = 0; k < P; k++) {
       const bool u = is_left(k);
       const float2 wu = u ? (k ? W[k - 1] : Wl) : W[k];
       const float2 gu = u ? (k ? G[k - 1] : Gl) : make_float2(-G[k].x, -G[k].y);
@@ -2521,8 +2532,8 @@ __device__ __forceinline__ void sweep_pass(float* sRr, int b0, const float (&v)[
     const float2 Fr = shdn2(F[0]);
     asm volatile("" ::: "memory");  // reread the rows rather than keep them in registers
 #pragma unroll
-    for (int k = 0; k < 8; k++) {
-      const float2 varq = s2(F[k], k < 7 ? F[k + 1] : Fr);
+    for (int k = 0; k < P; k++) {
+      const float2 varq = s2(F[k], k < P - 1 ? F[k + 1] : Fr);
       const float2 q = f2(varq, bc2(invsurf), make_float2(r0[k], r1[k]));  // unchanged rows: reread
       r0[k] = q.x;
       r1[k] = q.y;
@@ -2532,8 +2543,8 @@ __device__ __forceinline__ void sweep_pass(float* sRr, int b0, const float (&v)[
 
 // The residual and constant-residual van Leer sweeps of OneWindTheta
 // (StarThetaKernel, StarThetaKernel2, VanLeerThetaKernel, Kernels.cu:1157-1273)
-// on one ring's window of 256 points, by one warp: lane l holds points
-// 8l .. 8l+7 and takes its neighbours' edge values by shuffle.
+// on one ring's window of 32 P points, by one warp: lane l holds points
+// P l .. P l + P-1 and takes its neighbours' edge values by shuffle.
 // sRr: the ring's radial results [nq][kPad] and v_theta [kPad] (point x at
 // pidx(x)); the swept values go back to the same places.  The window's
 // points 0..3 and L-4.. (and any beyond L) are halo: each sweep's result at
@@ -2544,24 +2555,24 @@ __device__ __forceinline__ void sweep_pass(float* sRr, int b0, const float (&v)[
 // side for the whole ring (a warp-uniform branch), and none of it when that
 // residual is exactly zero (every flux is then zero: the quantities are
 // unchanged, as the reference's q + 0 leaves them).
-template <int nq>
+template <int nq, int P>
 __device__ __forceinline__ void sweep_ring(float* sRr, float VMed, float vconst, bool fast, float dt,
                                            float dxtheta, float invdxtheta, float invsurf, float dxrad) {
   const int lane = threadIdx.x & 31;
-  const int b0 = 9 * lane;  // pidx(8 * lane): points 8l .. 8l+7 are contiguous
-  float v[8];
+  const int b0 = (P + 1) * lane;  // pidx<P>(P * lane): a lane's points are contiguous
+  float v[P];
 #pragma unroll
-  for (int k = 0; k < 8; k++) {
-    float vres = sRr[nq * kPad + b0 + k] - VMed;
+  for (int k = 0; k < P; k++) {
+    float vres = sRr[nq * kPad<P> + b0 + k] - VMed;
     if (!fast) vres = vconst + vres;
     v[k] = vres;
   }
   if (!fast) vconst = 0.0f;
-  sweep_pass<nq, 0>(sRr, b0, v, 0.0f, dt, dxtheta, invdxtheta, invsurf, dxrad);
+  sweep_pass<nq, 0, P>(sRr, b0, v, 0.0f, dt, dxtheta, invdxtheta, invsurf, dxrad);
   if (fm(vconst, dt) > 0.0f)
-    sweep_pass<nq, 1>(sRr, b0, v, vconst, dt, dxtheta, invdxtheta, invsurf, dxrad);
+    sweep_pass<nq, 1, P>(sRr, b0, v, vconst, dt, dxtheta, invdxtheta, invsurf, dxrad);
   else if (vconst != 0.0f)
-    sweep_pass<nq, 2>(sRr, b0, v, vconst, dt, dxtheta, invdxtheta, invsurf, dxrad);
+    sweep_pass<nq, 2, P>(sRr, b0, v, vconst, dt, dxtheta, invdxtheta, invsurf, dxrad);
   __syncwarp();  // the ring's swept values, lane by lane, before the shifted store
 }
 
@@ -2573,8 +2584,8 @@ __device__ __forceinline__ void sweep_ring(float* sRr, float VMed, float vconst,
 // velocity vu for the whole ring (the constant-residual sweep), whose
 // interfaces all take their upwind value from the left (1: vu dt > 0) or
 // from the right (2), at the same distance h: no per-point selects.
-template <int nq, int kind>
-__device__ __forceinline__ void sweep_pass(float (&q)[nq][8], const float (&v)[8], float vu, float dt,
+template <int nq, int kind, int P>
+__device__ __forceinline__ void sweep_pass(float (&q)[nq][P], const float (&v)[P], float vu, float dt,
                                            float dxtheta, float invdxtheta, float invsurf, float dxrad) {
   auto slope = [&](float wm, float w0, float wp) -> float {
     float dqm = (w0 - wm);
@@ -2585,12 +2596,12 @@ __device__ __forceinline__ void sweep_pass(float (&q)[nq][8], const float (&v)[8
   };
   // upwind side of each point's left interface and the distance to it:
   // ksi > 0 takes point k-1 at dxtheta - ksi, else point k at -(dxtheta + ksi)
-  float vv[8], rr[8], S[8], GS[8], sD[8], h[8];
+  float vv[P], rr[P], S[P], GS[P], sD[P], h[P];
   unsigned up = 0;
   const float ksu = fm(vu, dt);
   const float hu = (kind == 1) ? dxtheta - ksu : dxtheta + ksu;
 #pragma unroll
-  for (int k = 0; k < 8; k++) {
+  for (int k = 0; k < P; k++) {
     vv[k] = (kind == 0) ? v[k] : vu;
     S[k] = q[nq - 1][k];
     rr[k] = rcp_ftz(S[k] + 1e-20f);
@@ -2603,14 +2614,14 @@ __device__ __forceinline__ void sweep_pass(float (&q)[nq][8], const float (&v)[8
     }
   }
   auto is_left = [&](int k) -> bool { return kind == 0 ? ((up >> k) & 1u) != 0 : kind == 1; };
-  const float Sl = __shfl_up_sync(0xffffffffu, S[7], 1);
+  const float Sl = __shfl_up_sync(0xffffffffu, S[P - 1], 1);
   const float Sr = __shfl_down_sync(0xffffffffu, S[0], 1);
 #pragma unroll
-  for (int k = 0; k < 8; k++) GS[k] = slope(k ? S[k - 1] : Sl, S[k], k < 7 ? S[k + 1] : Sr);
-  const float GSl = (kind == 2) ? 0.0f : __shfl_up_sync(0xffffffffu, GS[7], 1);
+  for (int k = 0; k < P; k++) GS[k] = slope(k ? S[k - 1] : Sl, S[k], k < P - 1 ? S[k + 1] : Sr);
+  const float GSl = (kind == 2) ? 0.0f : __shfl_up_sync(0xffffffffu, GS[P - 1], 1);
   // DensStar (StarThetaKernel2 on the density); a - fm(h, g) = a + fm(h, -g)
 #pragma unroll
-  for (int k = 0; k < 8; k++) {
+  for (int k = 0; k < P; k++) {
     const bool u = is_left(k);
     const float su = u ? (k ? S[k - 1] : Sl) : S[k];
     const float gu = u ? (k ? GS[k - 1] : GSl) : -GS[k];
@@ -2619,16 +2630,16 @@ __device__ __forceinline__ void sweep_pass(float (&q)[nq][8], const float (&v)[8
   // every quantity, density last; all quotients use the pre-sweep density
 #pragma unroll
   for (int c = 0; c < nq; c++) {
-    float W[8], G[8], F[8];
+    float W[P], G[P], F[P];
 #pragma unroll
-    for (int k = 0; k < 8; k++) W[k] = fm(q[c][k], rr[k]);
-    const float Wl = __shfl_up_sync(0xffffffffu, W[7], 1);
+    for (int k = 0; k < P; k++) W[k] = fm(q[c][k], rr[k]);
+    const float Wl = __shfl_up_sync(0xffffffffu, W[P - 1], 1);
     const float Wr = __shfl_down_sync(0xffffffffu, W[0], 1);
 #pragma unroll
-    for (int k = 0; k < 8; k++) G[k] = slope(k ? W[k - 1] : Wl, W[k], k < 7 ? W[k + 1] : Wr);
-    const float Gl = (kind == 2) ? 0.0f : __shfl_up_sync(0xffffffffu, G[7], 1);
+    for (int k = 0; k < P; k++) G[k] = slope(k ? W[k - 1] : Wl, W[k], k < P - 1 ? W[k + 1] : Wr);
+    const float Gl = (kind == 2) ? 0.0f : __shfl_up_sync(0xffffffffu, G[P - 1], 1);
 #pragma unroll
-    for (int k = 0; k < 8; k++) {
+    for (int k = 0; k < P; k++) {
       const bool u = is_left(k);
       const float wu = u ? (k ? W[k - 1] : Wl) : W[k];
       const float gu = u ? (k ? G[k - 1] : Gl) : -G[k];
@@ -2637,9 +2648,9 @@ __device__ __forceinline__ void sweep_pass(float (&q)[nq][8], const float (&v)[8
     }
     const float Fr = __shfl_down_sync(0xffffffffu, F[0], 1);
 #pragma unroll
-    for (int k = 0; k < 8; k++) {
+    for (int k = 0; k < P; k++) {
       float varq = F[k];
-      varq -= (k < 7 ? F[k + 1] : Fr);
+      varq -= (k < P - 1 ? F[k + 1] : Fr);
       q[c][k] += fm(varq, invsurf);
     }
   }
@@ -2647,8 +2658,8 @@ __device__ __forceinline__ void sweep_pass(float (&q)[nq][8], const float (&v)[8
 
 // The residual and constant-residual van Leer sweeps of OneWindTheta
 // (StarThetaKernel, StarThetaKernel2, VanLeerThetaKernel, Kernels.cu:1157-1273)
-// on one ring's window of 256 points, by one warp: lane l holds points
-// 8l .. 8l+7 in registers and takes its neighbours' edge values by shuffle.
+// on one ring's window of 32 P points, by one warp: lane l holds points
+// P l .. P l + P-1 in registers and takes its neighbours' edge values by shuffle.
 // sRr: the ring's radial results [nq][kPad] and v_theta [kPad] (point x at
 // pidx(x)); the swept values go back to the same places.  The window's
 // points 0..3 and L-4.. (and any beyond L) are halo: each sweep's result at
@@ -2659,31 +2670,31 @@ __device__ __forceinline__ void sweep_pass(float (&q)[nq][8], const float (&v)[8
 // side for the whole ring (a warp-uniform branch), and none of it when that
 // residual is exactly zero (every flux is then zero: the quantities are
 // unchanged, as the reference's q + 0 leaves them).
-template <int nq>
+template <int nq, int P>
 __device__ __forceinline__ void sweep_ring(float* sRr, float VMed, float vconst, bool fast, float dt,
                                            float dxtheta, float invdxtheta, float invsurf, float dxrad) {
   const int lane = threadIdx.x & 31;
-  const int b0 = 9 * lane;  // pidx(8 * lane): points 8l .. 8l+7 are contiguous
-  float q[nq][8], v[8];
+  const int b0 = (P + 1) * lane;  // pidx<P>(P * lane): a lane's points are contiguous
+  float q[nq][P], v[P];
 #pragma unroll
-  for (int k = 0; k < 8; k++) {
+  for (int k = 0; k < P; k++) {
 #pragma unroll
-    for (int c = 0; c < nq; c++) q[c][k] = sRr[c * kPad + b0 + k];
-    float vres = sRr[nq * kPad + b0 + k] - VMed;
+    for (int c = 0; c < nq; c++) q[c][k] = sRr[c * kPad<P> + b0 + k];
+    float vres = sRr[nq * kPad<P> + b0 + k] - VMed;
     if (!fast) vres = vconst + vres;
     v[k] = vres;
   }
   if (!fast) vconst = 0.0f;
-  sweep_pass<nq, 0>(q, v, 0.0f, dt, dxtheta, invdxtheta, invsurf, dxrad);
+  sweep_pass<nq, 0, P>(q, v, 0.0f, dt, dxtheta, invdxtheta, invsurf, dxrad);
   if (fm(vconst, dt) > 0.0f)
-    sweep_pass<nq, 1>(q, v, vconst, dt, dxtheta, invdxtheta, invsurf, dxrad);
+    sweep_pass<nq, 1, P>(q, v, vconst, dt, dxtheta, invdxtheta, invsurf, dxrad);
   else if (vconst != 0.0f)
-    sweep_pass<nq, 2>(q, v, vconst, dt, dxtheta, invdxtheta, invsurf, dxrad);
+    sweep_pass<nq, 2, P>(q, v, vconst, dt, dxtheta, invdxtheta, invsurf, dxrad);
   __syncwarp();
 #pragma unroll
-  for (int k = 0; k < 8; k++)
+  for (int k = 0; k < P; k++)
 #pragma unroll
-    for (int c = 0; c < nq; c++) sRr[c * kPad + b0 + k] = q[c][k];
+    for (int c = 0; c < nq; c++) sRr[c * kPad<P> + b0 + k] = q[c][k];
   __syncwarp();
 }
 
@@ -2855,13 +2866,13 @@ __device__ __forceinline__ void tr_fixup(const DiskDev& D, int4 it, float* sIn) 
 // k_ring_mean<1>.  Final density / energy go to scratch (a0 / a1) because
 // neighbouring bands still read the old ones; the velocity kernel moves
 // them into the state.
-template <int nq, bool solo>
+template <int nq, int P, bool solo>
 __global__ void __launch_bounds__(kTT, 2) k_transport(BatchDev B, const int4* __restrict__ items) {
   extern __shared__ __align__(16) float tr_sm[];
-  float* sR = tr_sm;                         // [kBR][nq + 1][kPad] radial results + v_theta
-  float* sL = sR + kBR * (nq + 1) * kPad;    // [kPad] mass through the inner edge (OPEN)
+  float* sR = tr_sm;                         // [kBR][nq + 1][kPad<P>] radial results + v_theta
+  float* sL = sR + kBR * (nq + 1) * kPad<P>;    // [kPad<P>] mass through the inner edge (OPEN)
   // [kInRows][kRow] staged input rows, 128-byte aligned (TMA destination)
-  float* sIn = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(sL + kPad) + 127) & ~uintptr_t(127));
+  float* sIn = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(sL + kPad<P>) + 127) & ~uintptr_t(127));
   __shared__ int s_jb[kBR];
   __shared__ float s_vmed[kBR], s_vc[kBR];
   __shared__ __align__(8) uint64_t s_bar;  // completion of the TMA staging
@@ -2924,25 +2935,32 @@ __global__ void __launch_bounds__(kTT, 2) k_transport(BatchDev B, const int4* __
       s_vmed[p] = D.tvmed[i0 + p];
       s_vc[p] = D.tvconst[i0 + p];
     }
-    if (p < L) {
-      const TrView V = {D.dens, D.vrad, D.vtheta, D.energy, D.Rmed, D.invdiffRmed, D.Rinf, D.Rsup, D.invSurf,
-                        nsec, nrad};
-      int g = (g0 - 4 + p) % nsec;
-      if (g < 0) g += nsec;
-      float* o = sR + pidx(p);
-      rad_march_s<nq>(V, sIn, i0, i0 + nb, p, g, dt, Om, dtheta, o, kPad, (nq + 1) * kPad,
-                      (D.OpenInner && i0 == 0) ? sL + pidx(p) : nullptr);
-      for (int r = 0; r < nb; r++) o[(r * (nq + 1) + nq) * kPad] = sIn[(kInT + r + 2) * kRow + p];
+    {
+      // P = 8: a column of the window per thread; 4: a column of half the band's rings
+      constexpr int NR = P == 8 ? kBR : kBR / 2;
+      const int k0 = P == 8 ? 0 : (p >> 7) * NR, col = P == 8 ? p : (p & 127);
+      if (col < L && k0 < nb) {
+        const TrView V = {D.dens, D.vrad, D.vtheta, D.energy, D.Rmed, D.invdiffRmed, D.Rinf, D.Rsup, D.invSurf,
+                          nsec, nrad};
+        int g = (g0 - 4 + col) % nsec;
+        if (g < 0) g += nsec;
+        const int ke = min(k0 + NR, nb);
+        float* o = sR + pidx<P>(col);
+        rad_march_s<nq, NR>(V, sIn + k0 * kRow, i0 + k0, i0 + ke, col, g, dt, Om, dtheta, o + k0 * (nq + 1) * kPad<P>,
+                            kPad<P>, (nq + 1) * kPad<P>, (D.OpenInner && i0 + k0 == 0) ? sL + pidx<P>(col) : nullptr,
+                            k0 + NR == kBR);
+        for (int r = k0; r < ke; r++) o[(r * (nq + 1) + nq) * kPad<P>] = sIn[(kInT + r + 2) * kRow + col];
+      }
     }
     __syncthreads();  // radial results complete; the staged rows are free
     if (tn < nai) pend = tr_stage<nq>(B, solo ? &sD : nullptr, items, tn, sIn, &s_bar);
     const int r = warp;
     if (r < nb) {
       const int i = i0 + r;
-      float* sRr = sR + (size_t)r * (nq + 1) * kPad;
+      float* sRr = sR + (size_t)r * (nq + 1) * kPad<P>;
       const float Rm = D.Rmed[i];
       const float dxtheta = fm(dtheta, Rm);
-      sweep_ring<nq>(sRr, s_vmed[r], s_vc[r], fast, dt, dxtheta, 1.0f / dxtheta, 1.0f / D.Surf[i],
+      sweep_ring<nq, P>(sRr, s_vmed[r], s_vc[r], fast, dt, dxtheta, 1.0f / dxtheta, 1.0f / D.Surf[i],
                      fm(D.Rsup[i] - D.Rinf[i], dt));
       // window point x is source sector g0 + x - 4, stored at output sector
       // jb + x - 4 (jb < nsec and x - 4 < S <= nsec: one wrap at most)
@@ -2953,8 +2971,8 @@ __global__ void __launch_bounds__(kTT, 2) k_transport(BatchDev B, const int4* __
         int j = jb + x;
         if (j >= nsec) j -= nsec;
 #pragma unroll
-        for (int c = 0; c < nq; c++) dsts[c == nq - 1 ? 5 : c][row + j] = sRr[c * kPad + pidx(x)];
-        if (i == 0 && D.OpenInner) D.lost[g0 + x - 4] = sL[pidx(x)];
+        for (int c = 0; c < nq; c++) dsts[c == nq - 1 ? 5 : c][row + j] = sRr[c * kPad<P> + pidx<P>(x)];
+        if (i == 0 && D.OpenInner) D.lost[g0 + x - 4] = sL[pidx<P>(x)];
       }
     }
   }
@@ -3755,6 +3773,16 @@ static void go(void (*kernel)(P...), int grid, int threads, size_t smem, cudaStr
   cudaLaunchKernelEx(&c, kernel, P(args)...);
 }
 
+template <int nq>
+static void launch_transport(const BatchDev& b, int nitems, const int4* items, cudaStream_t s, bool pdl) {
+  const bool solo = b.ndisk == 1;
+  const int grid = std::min(b.g_transport, nitems), adi = nq == 6;
+  if (b.tr_narrow)
+    go(INST(k_transport, nq, 4), grid, kTT, transport_smem_bytes<4>(adi), s, pdl, b, items);
+  else
+    go(INST(k_transport, nq, 8), grid, kTT, transport_smem_bytes<8>(adi), s, pdl, b, items);
+}
+
 void fargo_launch_substep(const BatchDev& b, cudaGraphConditionalHandle h, int use_handle, cudaStream_t s,
                           int max_nsec, long long* launches, cudaEvent_t* ev, int part, GraphBranch* sg) {
   (void)max_nsec;
@@ -3798,16 +3826,21 @@ void fargo_launch_substep(const BatchDev& b, cudaGraphConditionalHandle h, int u
   REC();
   if (sg) sg->join();  // the source terms read the accelerations
   bool chain = pdl && !sg;  // a kernel behind two branches waits for both in full
+  // Substep1 of a disk with NSEC no multiple of 4 keeps the general instance: in
+  // the other one the compiler contracts the pressure differences of the cell by
+  // cell path differently
+  const bool src1_solo = solo && !b.ragged;
+#define SRC1(adi, sg) (src1_solo ? k_source1<adi, sg, true> : k_source1<adi, sg, false>)
   if (b.any_bc) go(k_boundary<0>, b.ring_grid, kThreads, 0, s, std::exchange(chain, pdl), b);
   REC();
   if (b.src1_classes & 1)
-    go(INST(k_source1, 0, 0), b.g_source1[0], kThreads, 0, s, std::exchange(chain, pdl), b);
+    go(SRC1(0, 0), b.g_source1[0], kThreads, 0, s, std::exchange(chain, pdl), b);
   if (b.src1_classes & 2)
-    go(INST(k_source1, 0, 1), b.g_source1[1], kThreads, 0, s, std::exchange(chain, pdl), b);
+    go(SRC1(0, 1), b.g_source1[1], kThreads, 0, s, std::exchange(chain, pdl), b);
   if (b.src1_classes & 4)
-    go(INST(k_source1, 1, 0), b.g_source1[2], kThreads, 0, s, std::exchange(chain, pdl), b);
+    go(SRC1(1, 0), b.g_source1[2], kThreads, 0, s, std::exchange(chain, pdl), b);
   if (b.src1_classes & 8)
-    go(INST(k_source1, 1, 1), b.g_source1[3], kThreads, 0, s, std::exchange(chain, pdl), b);
+    go(SRC1(1, 1), b.g_source1[3], kThreads, 0, s, std::exchange(chain, pdl), b);
   REC();
   go((solo ? k_viscosity<true> : k_viscosity<false>), b.g_viscosity, kThreads, kViscSmem, s, pdl, b);
   REC();
@@ -3821,11 +3854,9 @@ void fargo_launch_substep(const BatchDev& b, cudaGraphConditionalHandle h, int u
   go(INST(k_ring_mean, 1), b.grp_grid, kRMT, fargo_ring_mean_smem_bytes(), s, pdl, b);
   REC();
   if (b.ntheta_iso)
-    go(INST(k_transport, 5), std::min(b.g_transport, b.ntheta_iso), kTT, fargo_transport_smem_bytes(0), s, pdl, b,
-       b.theta_iso);
+    launch_transport<5>(b, b.ntheta_iso, b.theta_iso, s, pdl);
   if (b.ntheta_adi)
-    go(INST(k_transport, 6), std::min(b.g_transport, b.ntheta_adi), kTT, fargo_transport_smem_bytes(1), s, pdl, b,
-       b.theta_adi);
+    launch_transport<6>(b, b.ntheta_adi, b.theta_adi, s, pdl);
   REC();
   const int last = solo && !b.any_bc;
   if (b.ntheta_iso) go(INST(k_velocities, 0), b.g_velocities[0], kThreads, 0, s, pdl, b, h, use_handle, last);
@@ -3836,6 +3867,7 @@ void fargo_launch_substep(const BatchDev& b, cudaGraphConditionalHandle h, int u
   if (fork && !last) branch.join();
   if (!last) go(k_substep_end, 1, kThreads, 0, s, pdl && !fork, b, h, use_handle);
   REC();
+#undef SRC1
 #undef REC
   if (launches) *launches += FARGO_KNS::fargo_substep_launches(b) - ((part & FARGO_PART_HEAD) ? 0 : 2);
 }
@@ -3853,13 +3885,8 @@ int fargo_launch_stripe_finish(const BatchDev& b, const double* blk, int nstripe
 // The transport kernels alone (both forms), for the autotuner: they read the
 // state and the last substep's ring means and write only scratch.
 void fargo_launch_transport(const BatchDev& b, cudaStream_t s) {
-  const bool solo = b.ndisk == 1;
-  if (b.ntheta_iso)
-    go(INST(k_transport, 5), std::min(b.g_transport, b.ntheta_iso), kTT,
-       fargo_transport_smem_bytes(0), s, false, b, b.theta_iso);
-  if (b.ntheta_adi)
-    go(INST(k_transport, 6), std::min(b.g_transport, b.ntheta_adi), kTT,
-       fargo_transport_smem_bytes(1), s, false, b, b.theta_adi);
+  if (b.ntheta_iso) launch_transport<5>(b, b.ntheta_iso, b.theta_iso, s, false);
+  if (b.ntheta_adi) launch_transport<6>(b, b.ntheta_adi, b.theta_adi, s, false);
 }
 
 // The CFL/force kernel instance for up to max_body bodies.
@@ -3895,7 +3922,7 @@ cudaError_t fargo_size_grids(BatchDev& b, int nsm, long long ncell_tiles, int ni
   if ((e = wave((const void*)k_energy<false>, kThreads, 0, ncell_tiles, &b.g_energy))) return e;
   if ((e = wave((const void*)k_velocities<0, false>, kThreads, 0, ncell_tiles, &b.g_velocities[0]))) return e;
   if ((e = wave((const void*)k_velocities<1, false>, kThreads, 0, ncell_tiles, &b.g_velocities[1]))) return e;
-  return wave((const void*)k_transport<6, false>, kTT, fargo_transport_smem_bytes(1), nitems, &b.g_transport);
+  return wave((const void*)k_transport<6, 8, false>, kTT, transport_smem_bytes<8>(1), nitems, &b.g_transport);
 }
 
 // Launches of one substep: 7 kernels (6 for one disk with rigid boundaries, whose
@@ -3939,10 +3966,14 @@ cudaError_t fargo_kernel_attributes(int max_nsec) {
   smem((const void*)k_ring_mean<1, true>, fargo_ring_mean_smem_bytes());
   smem((const void*)k_viscosity<false>, kViscSmem);
   smem((const void*)k_viscosity<true>, kViscSmem);
-  smem((const void*)k_transport<5, false>, fargo_transport_smem_bytes(0));
-  smem((const void*)k_transport<5, true>, fargo_transport_smem_bytes(0));
-  smem((const void*)k_transport<6, false>, fargo_transport_smem_bytes(1));
-  smem((const void*)k_transport<6, true>, fargo_transport_smem_bytes(1));
+  smem((const void*)k_transport<5, 8, false>, transport_smem_bytes<8>(0));
+  smem((const void*)k_transport<5, 4, false>, transport_smem_bytes<4>(0));
+  smem((const void*)k_transport<5, 8, true>, transport_smem_bytes<8>(0));
+  smem((const void*)k_transport<5, 4, true>, transport_smem_bytes<4>(0));
+  smem((const void*)k_transport<6, 8, false>, transport_smem_bytes<8>(1));
+  smem((const void*)k_transport<6, 4, false>, transport_smem_bytes<4>(1));
+  smem((const void*)k_transport<6, 8, true>, transport_smem_bytes<8>(1));
+  smem((const void*)k_transport<6, 4, true>, transport_smem_bytes<4>(1));
   return e;
 }
 
