@@ -3849,14 +3849,21 @@ void fargo_launch_substep(const BatchDev& b, cudaGraphConditionalHandle h, int u
   REC();
   if (b.any_bc) go(k_boundary<1>, b.ring_grid, kThreads, 0, s, pdl, b);
   REC();
-  if (b.ntheta_adi) go((solo ? k_energy<true> : k_energy<false>), b.g_energy, kThreads, 0, s, pdl, b);  // adiabatic disks only
+  // adiabatic disks only; in a graph beside the ring means, which read the
+  // velocities alone (201x602: 75.0 -> 70.3 us a substep, 1024x3072 343.0 -> 340.7,
+  // 256x768 64.5 -> 64.3; behind a boundary call the branch cost more than it
+  // gave, 113.9 -> 115.2)
+  GraphBranch heat;
+  const bool beside = b.ntheta_adi && !b.any_bc && heat.begin(s);
+  if (b.ntheta_adi) go((solo ? k_energy<true> : k_energy<false>), b.g_energy, kThreads, 0, s, pdl, b);
+  if (beside) heat.leave();
   REC();
   go(INST(k_ring_mean, 1), b.grp_grid, kRMT, fargo_ring_mean_smem_bytes(), s, pdl, b);
   REC();
-  if (b.ntheta_iso)
-    launch_transport<5>(b, b.ntheta_iso, b.theta_iso, s, pdl);
-  if (b.ntheta_adi)
-    launch_transport<6>(b, b.ntheta_adi, b.theta_adi, s, pdl);
+  if (beside) heat.join();
+  chain = pdl && !beside;
+  if (b.ntheta_iso) launch_transport<5>(b, b.ntheta_iso, b.theta_iso, s, std::exchange(chain, pdl));
+  if (b.ntheta_adi) launch_transport<6>(b, b.ntheta_adi, b.theta_adi, s, chain);
   REC();
   const int last = solo && !b.any_bc;
   if (b.ntheta_iso) go(INST(k_velocities, 0), b.g_velocities[0], kThreads, 0, s, pdl, b, h, use_handle, last);
