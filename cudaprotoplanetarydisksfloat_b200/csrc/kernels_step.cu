@@ -1547,26 +1547,17 @@ __device__ __forceinline__ Tau viscous_terms(const DiskDev& D, const float* Vr, 
   return t;
 }
 
-// Sub-Keplerian boundary speeds (SideEuler.cu:250-268), device double math
-// when they change with time or self-gravity.
-__device__ void vkep_pair(const DiskDev& D, const DiskCtl* C, float* vin, float* vout) {
-  if (D.vkep_const) {
-    *vin = D.VKepIn;
-    *vout = D.VKepOut;
-    return;
-  }
-  const int nrad = D.nrad;
+// Sub-Keplerian boundary speed (SideEuler.cu:250-268) at the inner (outer = 0)
+// or the outer edge ring, device double math when it changes with time or
+// self-gravity.
+__device__ float vkep_edge(const DiskDev& D, const DiskCtl* C, int outer) {
+  if (D.vkep_const) return outer ? D.VKepOut : D.VKepIn;
   float PT = C->time_start, PTI = C->PhysicalTimeInitial;
-  float r0 = D.Rmed[0], r1 = D.Rmed[nrad - 1];
+  float r = D.Rmed[outer ? D.nrad - 1 : 0];
   double f = (1.0 + D.SIGMASLOPE - 2.0 * D.FLARINGINDEX);
-  double a0 = 1.0 / r0 * (1.0 - f * pow((double)aspect_ratio_host(D, r0, PT, PTI), 2.0) * pow(r0, 2.0 * D.FLARINGINDEX));
-  double a1 = 1.0 / r1 * (1.0 - f * pow((double)aspect_ratio_host(D, r1, PT, PTI), 2.0) * pow(r1, 2.0 * D.FLARINGINDEX));
-  if (D.SelfGravity) {
-    a0 -= r0 * C->axisg_in;
-    a1 -= r1 * C->axisg_out;
-  }
-  *vin = sqrt(a0);
-  *vout = sqrt(a1);
+  double a = 1.0 / r * (1.0 - f * pow((double)aspect_ratio_host(D, r, PT, PTI), 2.0) * pow(r, 2.0 * D.FLARINGINDEX));
+  if (D.SelfGravity) a -= r * (outer ? C->axisg_out : C->axisg_in);
+  return sqrt(a);
 }
 
 // ComputeViscousTerms + UpdateVelocitiesWithViscosity + the sub-Keplerian
@@ -1621,6 +1612,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_viscosity(BatchDev B) {
   float(*sDnb)[kSR][kSC] = sVab + 2;
   __shared__ float sD0b[2][kSR];
   __shared__ float sTrr[kTR][kTCp], sTpp[kTR][kTCp], sTrp[kTR][kTCp];
+  __shared__ float s_vkep[2];
   const int tid = threadIdx.x;
   chain_start<solo>(B, &sD);
   const int na = solo ? 1 : B.act[0];
@@ -1687,6 +1679,17 @@ __global__ void __launch_bounds__(kThreads, 3) k_viscosity(BatchDev B) {
       have = false;
     }
     if (!have) stage(t - lo, bf);
+    // the edge speeds, by two threads while the staged rows arrive (two FP64
+    // powers: by every thread after the stresses they made 512x1024's edge tiles,
+    // and so the kernel, 14.1 instead of 12.5 us)
+    const int ncol = (sD.nsec + kVC - 1) / kVC;
+    const int lt = t - lo;
+    const int i0 = (lt / ncol) * kVR, j0 = (lt % ncol) * kVC;
+    const bool kep = !sD.Evanescent && (i0 == 0 || i0 + kVR >= sD.nrad);
+    if (kep && tid >= kThreads - 2) {
+      const int outer = tid - (kThreads - 2);
+      if (outer ? i0 + kVR >= sD.nrad : i0 == 0) s_vkep[outer] = vkep_edge(sD, sD.ctl, outer);
+    }
     // prefetch the next tile of the same disk while this one is computed
     const bool pre = (t + 1 < t1) && (t + 1 < hi);
     if (pre) {
@@ -1703,9 +1706,6 @@ __global__ void __launch_bounds__(kThreads, 3) k_viscosity(BatchDev B) {
     const DiskDev& D = sD;
     const DiskCtl* C = D.ctl;
     const int nsec = D.nsec, nrad = D.nrad;
-    const int ncol = (nsec + kVC - 1) / kVC;
-    const int lt = t - lo;
-    const int i0 = (lt / ncol) * kVR, j0 = (lt % ncol) * kVC;
     const float invdphi = D.invdphi, onethird = D.onethird;
     if (D.IsDisk) {
       // stresses at rows i0-1 .. i0+kVR, columns j0-1 .. j0+kVC (viscous_terms),
@@ -1764,9 +1764,6 @@ __global__ void __launch_bounds__(kThreads, 3) k_viscosity(BatchDev B) {
     __syncthreads();
     // updated velocities of the tile's cells: one quad per thread
     const float DeltaT = C->dtf;
-    float vin = 0.0f, vout = 0.0f;
-    const bool kep = !D.Evanescent && (i0 == 0 || i0 + kVR >= nrad);
-    if (kep) vkep_pair(D, C, &vin, &vout);
     {
       const int r = tid / (kVC / 4), c0 = 4 * (tid - r * (kVC / 4));
       const int i = i0 + r, j = j0 + c0;
@@ -1812,8 +1809,8 @@ __global__ void __launch_bounds__(kThreads, 3) k_viscosity(BatchDev B) {
                                          0.5f * (tpp0[u + 1] + tpp1[u])),
                                     0.5f * (dn[u + 1] + dnm[u]));
             }
-            if (kep && i == 0) vti[u] = vin - D.Rmed[0] * C->OmegaFrame;
-            if (kep && i == nrad - 1) vti[u] = vout - D.Rmed[nrad - 1] * C->OmegaFrame;
+            if (kep && i == 0) vti[u] = s_vkep[0] - D.Rmed[0] * C->OmegaFrame;
+            if (kep && i == nrad - 1) vti[u] = s_vkep[1] - D.Rmed[nrad - 1] * C->OmegaFrame;
           }
         }
         const int l = i * nsec + j;
