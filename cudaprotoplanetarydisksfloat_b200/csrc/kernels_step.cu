@@ -3,7 +3,7 @@
 // The reference runs ~120 single-purpose kernels, ~50 host-side reductions
 // (each with cudaMalloc/cudaFree) and ~15 full-grid device copies per
 // substep, with a device synchronisation after every launch
-// (SourceEuler.cu:230-299).  Here one substep of an isothermal batch is 10
+// (SourceEuler.cu:230-299).  Here one substep of an isothermal batch is 11
 // launches that read and write only the disk state and a few scratch fields,
 // with the CFL count, the disk forces and the planet integrator kept on the
 // device:
@@ -65,11 +65,29 @@ constexpr int kThreads = 256;
 // before it reads anything that a kernel writes.  (Launched without the
 // attribute, the wait is none.)  128x384: 61.0 -> 58.2 us a substep, 256x768
 // adiabatic 75.5 -> 72.5, 512x1536 105.1 -> 102.4, the 16-disk sweep 318 -> 313.
-// An earlier start is slower: let go at the start of the block before, the
-// waiting blocks of several kernels pile up on the SMs (67, 79, 102, 315 us); let
-// go after its wait, they hold the slots of the planets' and the self-gravity's
-// branches (57, 76, 101, 316 us).
+// An earlier start everywhere is slower: let go at the start of the block before,
+// the waiting blocks of several kernels pile up on the SMs (67, 79, 102, 315 us);
+// let go after its wait, they hold the slots of the planets' and the self-gravity's
+// branches (57, 76, 101, 316 us).  Where the next kernel has work of its own to do
+// meanwhile it pays: chain_release.
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// Lets the next kernel of the chain start now.  What that one does before its
+// wait may use only what was complete before this kernel passed its own wait, and
+// reads fields through L2.  Three places, each a few microseconds of serial work
+// that leaves most of the chip idle:
+//  - the ring means of the CFL (one disk): k_cfl_force loads its cells and forms
+//    the disk force, and waits before it reads the ring means;
+//  - the finish of the substep's scalars (one disk): k_potential forms the first
+//    planets' terms, and waits before it reads the indirect term;
+//  - the ring means of the transport (one isothermal disk): k_transport's first
+//    items are staged and marched radially before it reads the shifts.
+// The three together, us a substep: 64x192 47.6 -> 43.7, 128x384 50.5 -> 45.0, 512x1536
+// 97.7 -> 92.8, 512x1024 with self-gravity 113.8 -> 108.0, 256x768 adiabatic (the
+// first two) 65.3 -> 60.9, non-reflecting 116.2 -> 110.8, 1024x3072 343.8 -> 340.2.  A
+// batch keeps the waits at the start: its kernels fill the chip by themselves (16
+// disks 313 with any of the three).
+__device__ __forceinline__ void chain_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 __device__ __forceinline__ int disk_of_cell(const BatchDev& B, long long c) {
   int lo = 0, hi = B.ndisk - 1;
@@ -466,13 +484,15 @@ __device__ __forceinline__ void copy_words(void* dst, const void* src, int bytes
 // wait are the fields themselves, not a chain of four dependent loads (64x192:
 // 58.2 -> 56.0 us a substep, 256x768 adiabatic 72.7 -> 71.2; as a run-time choice in one
 // instance it cost the 16-disk sweep 1.5%).
-template <bool solo>
+// late (with solo): the caller waits later, on every path.
+template <bool solo, bool late = false>
 __device__ __forceinline__ void chain_start(const BatchDev& B, DiskDev* sD) {
+  static_assert(solo || !late, "the lists of active disks are read after the wait");
   if (solo) {
     copy_words(sD, B.disks, sizeof(DiskDev));
     __syncthreads();
   }
-  chain_wait();
+  if (!late) chain_wait();
 }
 
 // Four consecutive cells c0 .. c0+3 of one disk (c0 a multiple of 4).  With
@@ -495,10 +515,11 @@ struct Quad {
 // -1: any): only the disks whose Adiabatic / SelfGravity flags match (the
 // energy kernel takes adiabatic disks, the Substep1 instances one kind each).
 static_assert(FARGO_QTILE == 4 * kThreads, "four cells per thread");
-template <int kAdi, int kSg, bool solo, class Body>
+// late: the body waits for the previous kernel itself (chain_start).
+template <int kAdi, int kSg, bool solo, bool late, class Body>
 __device__ __forceinline__ void for_active_quads(const BatchDev& B, Body body) {
   __shared__ DiskDev sD;
-  chain_start<solo>(B, &sD);
+  chain_start<solo, late>(B, &sD);
   const int na = solo ? 1 : B.act[0];
   if (na <= 0) return;
   const int ntile = solo ? (int)(((long long)sD.nrad * sD.nsec + FARGO_QTILE - 1) / FARGO_QTILE) : B.act_tile_off[na];
@@ -643,8 +664,9 @@ __device__ __forceinline__ void qst(float* p, const Quad<V>& q, const float (&v)
   }
 }
 
-#define QUAD_BEGIN_T(kAdi, kSg)                                                                         \
-  for_active_quads<kAdi, kSg, solo>(B, [&](const DiskDev& D, const DiskCtl* C, const auto& q) {              \
+#define QUAD_BEGIN_T(kAdi, kSg) QUAD_BEGIN_L(kAdi, kSg, false)
+#define QUAD_BEGIN_L(kAdi, kSg, late)                                                                   \
+  for_active_quads<kAdi, kSg, solo, late>(B, [&](const DiskDev& D, const DiskCtl* C, const auto& q) {        \
     constexpr bool V = std::decay_t<decltype(q)>::vec;                                                 \
     (void)V;                                                                                           \
     const int nsec = D.nsec, nrad = D.nrad;                                                            \
@@ -778,7 +800,11 @@ constexpr int kRkShared = 16;  // planets whose RK5 scratch fits in shared memor
 
 // ConditionCFL host part (SourceEuler.cu:513-535): the shear limit DT1D
 // (ConditionCFLKernel2D2, Kernels.cu:1425-1428) of the ring pair (i, i+1).
+template <bool fresh>  // fresh: through L2, by a kernel that began before the means were done
 __device__ __forceinline__ float dt1d(const DiskDev& D, int i) {
+  if (fresh)
+    return 2.0 * PI_D * CFLSEC / (float)D.nsec /
+           fabsf(__ldcg(D.vmoy + i) * D.invRmed[i] - __ldcg(D.vmoy + i + 1) * D.invRmed[i + 1]);
   return 2.0 * PI_D * CFLSEC / (float)D.nsec / fabsf(D.vmoy[i] * D.invRmed[i] - D.vmoy[i + 1] * D.invRmed[i + 1]);
 }
 
@@ -1042,7 +1068,7 @@ __global__ void __launch_bounds__(kThreads, NB <= 1 ? 3 : 2) k_cfl_force(BatchDe
   __shared__ unsigned s_ticket;
   __shared__ int s_nbody;
   const int tid = threadIdx.x, w = tid >> 5, l = tid & 31;
-  chain_start<solo>(B, &sD);
+  chain_start<solo, solo>(B, &sD);
   const int na = solo ? 1 : B.act[0];
   const int ntile = solo ? fargo_cfl_tiles_own(sD) : na > 0 ? B.act_ctile_off[na] : 0;
   const int per = (ntile + gridDim.x - 1) / gridDim.x;
@@ -1067,6 +1093,7 @@ __global__ void __launch_bounds__(kThreads, NB <= 1 ? 3 : 2) k_cfl_force(BatchDe
     const int nct = fargo_cfl_tiles_own(sD);
     if (s_ticket + (unsigned)run == (unsigned)nct) {
       __threadfence();
+      if (solo) chain_release();
       finish_substep(sD, Cr, s_min[0], s_part, DiskTiles{sD, nct});
     }
     run = 0;
@@ -1109,11 +1136,11 @@ __global__ void __launch_bounds__(kThreads, NB <= 1 ? 3 : 2) k_cfl_force(BatchDe
       const int kh = D.ExcludeHill ? FARGO_DIMFXY - 1 : 0;
       const float hillcutfactor = (float)kh / (float)(FARGO_DIMFXY - 1);
       const int iend = D.own_hi;
-      // One cell (ring ic, sector cj): its CFL limit (rings > 0) and its
-      // force on every body.  Ring constants come in rt (dxrad, dxtheta,
-      // their three reciprocals, the ring-mean velocity, Rmed, Surf).
-      auto cell = [&](int ic, int cj, float v0, float vr0, float dn, float vrp, float vtp, float csv, float cth,
-                      float sth, const float (&rt)[8]) {
+      // One cell of ring ic: its CFL limit (rings > 0) and its force on every
+      // body.  Ring constants come in rt (dxrad, dxtheta, their three
+      // reciprocals, the ring-mean velocity, Rmed, Surf).
+      auto limit = [&](int ic, float v0, float vr0, float dn, float vrp, float vtp, float csv,
+                       const float (&rt)[8]) {
         // a NaN or Inf in the state: a NaN dt2d would be skipped by the
         // minimum below (as the reference's is) and the step would go on
         // with it; mark the tile instead, so that the DT stops with
@@ -1147,8 +1174,9 @@ __global__ void __launch_bounds__(kThreads, NB <= 1 ? 3 : 2) k_cfl_force(BatchDe
               0.5f * __frcp_rn(sqrtf(invdt1 * invdt1 + invdt2 * invdt2 + invdt3 * invdt3 + invdt4 * invdt4));
           if (dt2d < lmin) lmin = dt2d;
         }
-        const float Rm = rt[6];
-        float cellmass = rt[7] * dn;
+      };
+      auto force = [&](float dn, float cth, float sth, float Rm, float surf) {
+        float cellmass = surf * dn;
         float cx = Rm * cth;
         float cy = Rm * sth;
 #pragma unroll
@@ -1180,11 +1208,17 @@ __global__ void __launch_bounds__(kThreads, NB <= 1 ? 3 : 2) k_cfl_force(BatchDe
           }
         }
       };
+      auto cell = [&](int ic, float v0, float vr0, float dn, float vrp, float vtp, float csv, float cth, float sth,
+                      const float (&rt)[8]) {
+        limit(ic, v0, vr0, dn, vrp, vtp, csv, rt);
+        force(dn, cth, sth, rt[6], rt[7]);
+      };
+      auto state = [](const auto* p) { return solo ? __ldcg(p) : __ldg(p); };
       // once per ring: the shear limit of the pair (i, i+1), and FViscosity for
       // this substep (Viscosity.cu:84-85, SourceEuler.cu:350)
       auto ring = [&](int i) {
         if (i < nrad - 1) {
-          const float dt1 = dt1d(D, i);
+          const float dt1 = dt1d<solo>(D, i);
           if (dt1 < lmin) lmin = dt1;
         }
         if (!D.stripe) D.visc[i] = fviscosity_ring(D, i, D.ctl->PhysicalTime, D.ctl->PhysicalTimeInitial);
@@ -1195,7 +1229,7 @@ __global__ void __launch_bounds__(kThreads, NB <= 1 ? 3 : 2) k_cfl_force(BatchDe
         rt[2] = D.cfl_rdr[ic];
         rt[3] = D.cfl_rdt[ic];
         rt[4] = D.cfl_rmd[ic];
-        rt[5] = D.FastTransport ? D.vmoy[ic] : 0.0f;
+        rt[5] = !D.FastTransport ? 0.0f : solo ? __ldcg(D.vmoy + ic) : D.vmoy[ic];
         rt[6] = D.Rmed[ic];
         rt[7] = D.Surf[ic];
       };
@@ -1210,22 +1244,39 @@ __global__ void __launch_bounds__(kThreads, NB <= 1 ? 3 : 2) k_cfl_force(BatchDe
         for (int g = 0; g < nq; g++) {
           if (i >= iend) break;
           const int q = i * nsec + j;
-          const float4 V0 = __ldg(reinterpret_cast<const float4*>(D.vtheta + q));
-          const float4 VR0 = __ldg(reinterpret_cast<const float4*>(D.vrad + q));
-          const float4 DN = __ldg(reinterpret_cast<const float4*>(D.dens + q));
-          const float4 VRP = __ldg(reinterpret_cast<const float4*>(D.vrad + q + nsec));
-          const float vt4 = __ldg(D.vtheta + q - j + (j + 4 == nsec ? 0 : j + 4));
-          const float4 CS = D.Adiabatic ? __ldg(reinterpret_cast<const float4*>(D.cs + q))
+          const float4 V0 = state(reinterpret_cast<const float4*>(D.vtheta + q));
+          const float4 VR0 = state(reinterpret_cast<const float4*>(D.vrad + q));
+          const float4 DN = state(reinterpret_cast<const float4*>(D.dens + q));
+          const float4 VRP = state(reinterpret_cast<const float4*>(D.vrad + q + nsec));
+          const float vt4 = state(D.vtheta + q - j + (j + 4 == nsec ? 0 : j + 4));
+          const float4 CS = D.Adiabatic ? state(reinterpret_cast<const float4*>(D.cs + q))
                                         : make_float4(D.cs_ring[i], D.cs_ring[i], D.cs_ring[i], D.cs_ring[i]);
           const float4 CT = __ldg(reinterpret_cast<const float4*>(D.cos_cell + j));
           const float4 ST = __ldg(reinterpret_cast<const float4*>(D.sin_cell + j));
           float rt[8];
-          ring_consts(i, rt);
-          if (j == 0) ring(i);
-          cell(i, j, V0.x, VR0.x, DN.x, VRP.x, V0.y, CS.x, CT.x, ST.x, rt);
-          cell(i, j + 1, V0.y, VR0.y, DN.y, VRP.y, V0.z, CS.y, CT.y, ST.y, rt);
-          cell(i, j + 2, V0.z, VR0.z, DN.z, VRP.z, V0.w, CS.z, CT.z, ST.z, rt);
-          cell(i, j + 3, V0.w, VR0.w, DN.w, VRP.w, vt4, CS.w, CT.w, ST.w, rt);
+          if (solo) {
+            // the forces need no ring mean: in the block's first step they are
+            // formed while the ring means are
+            const float Rm = D.Rmed[i], surf = D.Surf[i];
+            force(DN.x, CT.x, ST.x, Rm, surf);
+            force(DN.y, CT.y, ST.y, Rm, surf);
+            force(DN.z, CT.z, ST.z, Rm, surf);
+            force(DN.w, CT.w, ST.w, Rm, surf);
+            if (g == 0) chain_wait();
+            ring_consts(i, rt);
+            if (j == 0) ring(i);
+            limit(i, V0.x, VR0.x, DN.x, VRP.x, V0.y, CS.x, rt);
+            limit(i, V0.y, VR0.y, DN.y, VRP.y, V0.z, CS.y, rt);
+            limit(i, V0.z, VR0.z, DN.z, VRP.z, V0.w, CS.z, rt);
+            limit(i, V0.w, VR0.w, DN.w, VRP.w, vt4, CS.w, rt);
+          } else {
+            ring_consts(i, rt);
+            if (j == 0) ring(i);
+            cell(i, V0.x, VR0.x, DN.x, VRP.x, V0.y, CS.x, CT.x, ST.x, rt);
+            cell(i, V0.y, VR0.y, DN.y, VRP.y, V0.z, CS.y, CT.y, ST.y, rt);
+            cell(i, V0.z, VR0.z, DN.z, VRP.z, V0.w, CS.z, CT.z, ST.z, rt);
+            cell(i, V0.w, VR0.w, DN.w, VRP.w, vt4, CS.w, CT.w, ST.w, rt);
+          }
           j += 4 * kThreads;
           while (j >= nsec) {
             j -= nsec;
@@ -1233,6 +1284,7 @@ __global__ void __launch_bounds__(kThreads, NB <= 1 ? 3 : 2) k_cfl_force(BatchDe
           }
         }
       } else {
+        if (solo) chain_wait();
         const int c0 = D.own_lo * nsec + k * D.cfl_tile + tid;
         int i = c0 / nsec, j = c0 - i * nsec;
         const int ncell = D.cfl_tile / kThreads;
@@ -1273,11 +1325,12 @@ __global__ void __launch_bounds__(kThreads, NB <= 1 ? 3 : 2) k_cfl_force(BatchDe
             float rt[8];
             ring_consts(ci[u], rt);
             if (cj[u] == 0) ring(ci[u]);
-            cell(ci[u], cj[u], v0[u], vr0[u], dn[u], vrp[u], vtp[u], csv[u], cth[u], sth[u], rt);
+            cell(ci[u], v0[u], vr0[u], dn[u], vrp[u], vtp[u], csv[u], cth[u], sth[u], rt);
           }
         }
       }
     }
+    if (solo) chain_wait();  // threads without a cell, and no disk
     // tile minimum and force sums: warps by shuffle, then warp 0 over the
     // warps (buffers alternate by tile, so one barrier per tile suffices)
     const int pb = t & 1;
@@ -1377,9 +1430,14 @@ __global__ void __launch_bounds__(kThreads) k_stripe_finish(BatchDev B, const do
 // per substep (Substep1 reads it at three cells each), summed over the
 // planets in the reference's order (FillForcesArraysKernel,
 // Kernels.cu:1322-1349); each planet's parameters are read once per quad.
-template <bool solo>
+// early (one disk, a tile per block at most): the terms of the first kEarly
+// bodies of the star's system are formed before the wait for k_cfl_force, which
+// then still finishes the substep's scalars; the sum keeps its order.  Its 16 more
+// registers cost a larger disk more than the overlap gives (1024x3072: 340.8 ->
+// 349.4 us a substep).  64x192 50.0 -> 48.7, 256x768 adiabatic 64.0 -> 62.9.
+template <bool solo, bool early>
 __global__ void __launch_bounds__(kThreads) k_potential(BatchDev B) {
-  QUAD_BEGIN
+  QUAD_BEGIN_L(-1, -1, early)
   float cp[4], sp[4], x[4], y[4], P[4];
   qld_sector(cp, D.cos_pot, q);
   qld_sector(sp, D.sin_pot, q);
@@ -1392,32 +1450,54 @@ __global__ void __launch_bounds__(kThreads) k_potential(BatchDev B) {
   }
   const int nb = C->nb;
   const bool ind = D.Indirect_Term;
-  for (int k = 0; k < nb; k++) {
-    const float xp = C->pxp[k], yp = C->pyp[k], mp = C->pmass[k], sm = C->psmooth[k], ip3 = C->pipd3[k];
+  auto term = [&](int u, float xp, float yp, float mp, float sm, float ip3) -> float {
+    float distance = (x[u] - xp) * (x[u] - xp) + (y[u] - yp) * (y[u] - yp);
+    float distancesmooth = sqrtf(distance + sm);
+    float pot = div_refined(-mp, distancesmooth);  // -G*mplanet/distancesmooth
+    if (ind) pot += mp * ip3 * (x[u] * xp + y[u] * yp);
+    return pot;
+  };
+  constexpr int kEarly = early ? 4 : 0;
+  float pe[kEarly + 1][4];
+  if (early) {
+#pragma unroll
+    for (int k = 0; k < kEarly; k++) {
+      if (k >= nb) break;
+      const float xp = C->pxp[k], yp = C->pyp[k], mp = C->pmass[k], sm = C->psmooth[k], ip3 = C->pipd3[k];
+#pragma unroll
+      for (int u = 0; u < 4; u++) pe[k][u] = term(u, xp, yp, mp, sm, ip3);
+    }
+    chain_wait();
+  }
+  auto star_term = [&]() {
+    const float itx = early ? __ldcg(&C->itx) : C->itx, ity = early ? __ldcg(&C->ity) : C->ity;
+    // accurate mode: the star's -G/r enters Substep1 as its exact radial
+    // difference quotient (star_grad) instead of a difference of FP32 values
+    const bool star = !D.accurate;
 #pragma unroll
     for (int u = 0; u < 4; u++) {
-      float distance = (x[u] - xp) * (x[u] - xp) + (y[u] - yp) * (y[u] - yp);
-      float distancesmooth = sqrtf(distance + sm);
-      float pot = div_refined(-mp, distancesmooth);  // -G*mplanet/distancesmooth
-      if (ind) pot += mp * ip3 * (x[u] * xp + y[u] * yp);
+      float InvDistance = __fdiv_rn(1.0f, D.Rmed[q.i[u]]);
+      float pot = star ? -InvDistance : 0.0f;
+      pot -= itx * x[u] + ity * y[u];
       P[u] += pot;
     }
-    if (k == 0) {  // the star
-      const float itx = C->itx, ity = C->ity;
-      // accurate mode: the star's -G/r enters Substep1 as its exact radial
-      // difference quotient (star_grad) instead of a difference of FP32 values
-      const bool star = !D.accurate;
+  };
 #pragma unroll
-      for (int u = 0; u < 4; u++) {
-        float InvDistance = __fdiv_rn(1.0f, D.Rmed[q.i[u]]);
-        float pot = star ? -InvDistance : 0.0f;
-        pot -= itx * x[u] + ity * y[u];
-        P[u] += pot;
-      }
-    }
+  for (int k = 0; k < kEarly; k++) {
+    if (k >= nb) break;
+#pragma unroll
+    for (int u = 0; u < 4; u++) P[u] += pe[k][u];
+    if (k == 0) star_term();
+  }
+  for (int k = kEarly; k < nb; k++) {
+    const float xp = C->pxp[k], yp = C->pyp[k], mp = C->pmass[k], sm = C->psmooth[k], ip3 = C->pipd3[k];
+#pragma unroll
+    for (int u = 0; u < 4; u++) P[u] += term(u, xp, yp, mp, sm, ip3);
+    if (k == 0) star_term();
   }
   qst(D.phi, q, P);
   QUAD_END
+  if (early) chain_wait();  // blocks and threads without a quad
 }
 
 // Substep1KernelVrad / Substep1KernelVtheta (Kernels.cu:52-88), with
@@ -2284,6 +2364,7 @@ __global__ void __launch_bounds__(kRMT) k_ring_mean(BatchDev B) {
   extern __shared__ __align__(16) float rm_sm[];  // [2][kRMR][kRMS]
   __shared__ DiskDev sD;  // a batch of one disk
   chain_start<solo>(B, &sD);
+  if (solo) chain_release();
   const int na = solo ? 1 : B.act[0];
   const int ng = solo ? (sD.nrad + kRMR - 1) / kRMR : na > 0 ? B.act_grp_off[na] : 0;
   const int tid = threadIdx.x, lane = tid & 31;
@@ -2818,6 +2899,7 @@ __device__ __forceinline__ bool tr_stage(const BatchDev& B, const DiskDev* solo,
 // not wrap); fill them from the other end of the ring, as the reference's
 // periodic azimuth reads them.  At most 4 columns on the left and 5 on the
 // right (the segment lies inside the ring).
+template <bool early>
 __device__ __forceinline__ void tr_fixup(const DiskDev& D, int4 it, float* sIn) {
   const int i0 = it.y, g0 = it.z, W = it.w + 9;
   const int nsec = D.nsec, nrad = D.nrad;
@@ -2844,7 +2926,8 @@ __device__ __forceinline__ void tr_fixup(const DiskDev& D, int4 it, float* sIn) 
       lim = nrad - 1;
       base = D.vtheta;
     }
-    sIn[row * kRow + c] = (r >= 0 && r <= lim) ? __ldg(base + r * nsec + g) : 0.0f;
+    const float* src = base + r * nsec + g;
+    sIn[row * kRow + c] = (r >= 0 && r <= lim) ? (early ? __ldcg(src) : __ldg(src)) : 0.0f;
   }
 }
 
@@ -2881,7 +2964,11 @@ __global__ void __launch_bounds__(kTT, 2) k_transport(BatchDev B, const int4* __
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     s_gaveup = 0;
   }
-  chain_start<solo>(B, &sD);
+  // one isothermal disk: the first items' radial half runs beside the ring means
+  // (the energy of an adiabatic disk is read outside the staged rows)
+  constexpr bool early = solo && nq == 5;
+  chain_start<solo, early>(B, &sD);
+  if (early && B.ragged) chain_wait();
   const int nak = solo ? 1 : (nq == 5) ? B.act[1] : B.act[2];
   const int* aoff = (nq == 5) ? B.act_iso_off : B.act_adi_off;
   const int* adisk = (nq == 5) ? B.act_iso_disk : B.act_adi_disk;
@@ -2897,7 +2984,7 @@ __global__ void __launch_bounds__(kTT, 2) k_transport(BatchDev B, const int4* __
     const int4 it = items[D.item0 + (solo ? t : t - aoff[a])];
     if (pend) {
       if (mbar_wait_bounded(&s_bar, phase)) {
-        tr_fixup(D, it, sIn);
+        tr_fixup<early>(D, it, sIn);
       } else {
         s_gaveup = 1;
       }
@@ -2909,6 +2996,7 @@ __global__ void __launch_bounds__(kTT, 2) k_transport(BatchDev B, const int4* __
       // it to FARGO_ETIMEOUT), wait once more for the copies, and stop
       if (p == 0) const_cast<DiskCtl*>(D.ctl)->error = 3;
       mbar_wait_bounded(&s_bar, phase);
+      if (early) chain_wait();
       return;
     }
     if (pend) phase ^= 1;
@@ -2926,12 +3014,15 @@ __global__ void __launch_bounds__(kTT, 2) k_transport(BatchDev B, const int4* __
     const float Om = C->OmegaFrame;
     const bool fast = D.FastTransport;
     const float dtheta = 2.0f * (float)PI_D / (float)nsec;
-    if (p < nb) {
-      int jb = (g0 + D.nshift[i0 + p]) % nsec;  // output sector of source sector g0
+    auto shifts = [&]() {
+      if (p >= nb) return;
+      const int ns = early ? __ldcg(D.nshift + i0 + p) : D.nshift[i0 + p];
+      int jb = (g0 + ns) % nsec;  // output sector of source sector g0
       s_jb[p] = jb < 0 ? jb + nsec : jb;
-      s_vmed[p] = D.tvmed[i0 + p];
-      s_vc[p] = D.tvconst[i0 + p];
-    }
+      s_vmed[p] = early ? __ldcg(D.tvmed + i0 + p) : D.tvmed[i0 + p];
+      s_vc[p] = early ? __ldcg(D.tvconst + i0 + p) : D.tvconst[i0 + p];
+    };
+    if (!early) shifts();
     {
       // P = 8: a column of the window per thread; 4: a column of half the band's rings
       constexpr int NR = P == 8 ? kBR : kBR / 2;
@@ -2948,6 +3039,10 @@ __global__ void __launch_bounds__(kTT, 2) k_transport(BatchDev B, const int4* __
                             k0 + NR == kBR);
         for (int r = k0; r < ke; r++) o[(r * (nq + 1) + nq) * kPad<P>] = sIn[(kInT + r + 2) * kRow + col];
       }
+    }
+    if (early) {
+      chain_wait();
+      shifts();
     }
     __syncthreads();  // radial results complete; the staged rows are free
     if (tn < nai) pend = tr_stage<nq>(B, solo ? &sD : nullptr, items, tn, sIn, &s_bar);
@@ -2973,6 +3068,7 @@ __global__ void __launch_bounds__(kTT, 2) k_transport(BatchDev B, const int4* __
       }
     }
   }
+  if (early) chain_wait();  // blocks without an item
   cp_async_wait<0>();
 }
 
@@ -3812,7 +3908,9 @@ void fargo_launch_substep(const BatchDev& b, cudaGraphConditionalHandle h, int u
     return;
   }
   REC();
-  go((solo ? k_potential<true> : k_potential<false>), b.g_potential, kThreads, 0, s, pdl && (part & FARGO_PART_HEAD), b);
+  // a block of the early form has one tile at most (one disk's cells per quad tile)
+  const bool ahead = solo && (b.ncell + FARGO_QTILE - 1) / FARGO_QTILE <= b.g_potential;
+  go((ahead ? k_potential<true, true> : solo ? k_potential<true, false> : k_potential<false, false>), b.g_potential, kThreads, 0, s, pdl && (part & FARGO_PART_HEAD), b);
   REC();
   // inside a graph the planets run beside the rest of the substep, unless its
   // kernels read the new frame
@@ -3919,7 +4017,7 @@ cudaError_t fargo_size_grids(BatchDev& b, int nsm, long long ncell_tiles, int ni
   if ((e = wave((const void*)k_source1<0, 1, false>, kThreads, 0, ncell_tiles, &b.g_source1[1]))) return e;
   if ((e = wave((const void*)k_source1<1, 0, false>, kThreads, 0, ncell_tiles, &b.g_source1[2]))) return e;
   if ((e = wave((const void*)k_source1<1, 1, false>, kThreads, 0, ncell_tiles, &b.g_source1[3]))) return e;
-  if ((e = wave((const void*)k_potential<false>, kThreads, 0, ncell_tiles, &b.g_potential))) return e;
+  if ((e = wave((const void*)k_potential<false, false>, kThreads, 0, ncell_tiles, &b.g_potential))) return e;
   if ((e = wave((const void*)k_viscosity<false>, kThreads, kViscSmem, ncell_tiles, &b.g_viscosity))) return e;
   if ((e = wave((const void*)k_source2<0, false>, kThreads, 0, ncell_tiles, &b.g_source2[0]))) return e;
   if ((e = wave((const void*)k_source2<1, false>, kThreads, 0, ncell_tiles, &b.g_source2[1]))) return e;
