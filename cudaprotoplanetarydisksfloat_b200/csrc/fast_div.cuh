@@ -20,6 +20,14 @@ __device__ __forceinline__ float div_by_recip(float x, float d, float r) {
   return __fmaf_rn(e, r, q0);
 }
 
+// The same where the quotient may overflow: there the correction would be
+// inf - inf = NaN, and the quotient is the infinity itself.
+__device__ __forceinline__ float div_by_recip_inf(float x, float d, float r) {
+  const float q0 = __fmul_rn(x, r);
+  const float q = __fmaf_rn(__fmaf_rn(-q0, d, x), r, q0);
+  return isinf(q0) ? q0 : q;
+}
+
 // x / d in double from r = RN(1/d) (Markstein's method as in div_by_recip):
 // the correctly rounded quotient for normal operands, in three operations.
 __device__ __forceinline__ double div_by_recip_d(double x, double d, double r) {

@@ -3750,7 +3750,8 @@ __global__ void __launch_bounds__(kThreads, 2) k_disk_force(BatchDev B, int disk
 #pragma unroll
       for (int k = 0; k < K; k++) {
         float hill_cut = 1.0f;
-        if (k != 0) hill_cut = 1. - expf(div_by_recip(-d2, rh2[k], ir2[k]));
+        // (a body without mass or at the origin has a cut radius of 1e-15)
+        if (k != 0) hill_cut = 1. - expf(div_by_recip_inf(-d2, rh2[k], ir2[k]));
         const float fx = px * hill_cut, fy = py * hill_cut;
         sx[k] += fx;
         sy[k] += fy;
