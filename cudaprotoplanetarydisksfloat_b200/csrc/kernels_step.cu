@@ -3496,9 +3496,10 @@ __global__ void __launch_bounds__(kThreads) k_boundary(BatchDev B) {
     t = te;
     if (!D.IsDisk) continue;
     const bool cs_rings = D.NonReflecting && D.Adiabatic;
+    const bool rings = cs_rings || D.Evanescent;
     const float dtf = C->dtf, domega = C->domega, OmegaFrame = C->OmegaFrame;
     const float time_start = C->time_start, PTI = C->PhysicalTimeInitial;
-    for (int i = first - lo; (cs_rings || D.Evanescent) && i < te - lo; i++) {
+    for (int i = first - lo; rings && i < te - lo; i++) {
       const size_t r0 = (size_t)i * nsec;
       if (cs_rings) {
         float sum = 0.0f;  // Make1DprofileKernel: sectors in order
@@ -3602,9 +3603,9 @@ __global__ void __launch_bounds__(kThreads) k_boundary(BatchDev B) {
       }
     }
     if (!(D.OpenInner || D.NonReflecting)) continue;
-    // the edge rings: after every ring's sound speed where there is one (the
+    // the edge rings: after every ring's own part where there is one (the
     // disk's ticket), else at once by the block of ring 0
-    if (cs_rings) {
+    if (rings) {
       __threadfence();
       __syncthreads();
       if (tid == 0) s_ticket = atomicAdd(&C->counter, (unsigned)run);
