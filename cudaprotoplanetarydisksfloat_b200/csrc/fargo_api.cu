@@ -804,6 +804,12 @@ fargo_status finish_dts(fargo_batch* b) {
   for (int d = 0; d < (int)b->disks.size(); d++) {
     const DiskCtl& c = b->h_ctl[d];
     if (c.error == 1) return set_err(b, FARGO_ENONFINITE, "disk %d: non-finite or non-positive CFL time step", d);
+    if (c.error == 4)
+      return set_err(b, FARGO_EINVAL,
+                     "disk %d: the non-reflecting boundary's angular offset leaves the grid (too few rings, or a "
+                     "vanishing sound speed)", d);
+    if (c.error == 5)
+      return set_err(b, FARGO_ENONFINITE, "disk %d: non-finite sound speed at a non-reflecting edge", d);
     if (c.error == 3)
       return set_err(b, FARGO_ETIMEOUT, "disk %d: a transport block gave up waiting for its staged rows", d);
     if (c.error == 2)

@@ -39,7 +39,7 @@ struct DiskCtl {
   int more;            // set by the CFL finalize: another substep follows
   int nsub;            // substeps taken in the current DT
   int nsub_total;
-  int error;           // nonzero: 1 non-finite CFL, 2 too many substeps
+  int error;           // nonzero: 1 non-finite CFL, 2 too many substeps, 3 a bounded wait, 4 / 5 edge offsets (bc_offset.h)
   unsigned int counter;        // last-block ticket of the CFL/force kernel
   float PhysicalTime;          // advanced at the end of each substep
   float time_start;            // PhysicalTime at the start of this substep

@@ -49,6 +49,7 @@
 #include <type_traits>
 #include <utility>
 
+#include "bc_offset.h"
 #include "fargo_internal.h"
 #include "fast_div.cuh"
 
@@ -3327,7 +3328,7 @@ __global__ void k_cs_ringmean(BatchDev B, int only_disk) {
 // The sound speed may have been written by other blocks of this launch: it is
 // read through L2.  sm: 4 * kThreads floats.
 __device__ void boundary_edges(const DiskDev& D, float* sm) {
-  __shared__ int s_angle[2];
+  __shared__ int s_angle[2], s_reach;
   const int tid = threadIdx.x;
   const int nsec = D.nsec, nrad = D.nrad;
   float* Dn = D.dens;
@@ -3358,34 +3359,37 @@ __device__ void boundary_edges(const DiskDev& D, float* sm) {
       // host arithmetic of NonReflectingBoundary, pow() of the radii from the host
       double dangle = (D.nr_pow_in - 1.0) / (.5 * (cs0_r + cs1_r));
       dangle *= (D.Rmed[1] - D.Rmed[0]);
-      s_angle[0] = (int)(dangle / 2.0 / PI_D * (float)nsec + .5);
+      const double off = dangle / 2.0 / PI_D * (float)nsec + .5;
       double dangle2 = (D.nr_pow_out - 1.0) / (.5 * (csnrm1_r + csnrm2_r));
       dangle2 *= (D.Rmed[nrad - 1] - D.Rmed[nrad - 2]);
-      s_angle[1] = (int)(dangle2 / 2.0 / PI_D * (float)nsec + .5);
+      const double off2 = dangle2 / 2.0 / PI_D * (float)nsec + .5;
+      s_reach = bc_reach(off, off2, nrad, nsec);
+      s_angle[0] = s_reach <= kBcInRows ? (int)off : 0;
+      s_angle[1] = s_reach <= kBcInRows ? (int)off2 : 0;
+      if (s_reach > kBcInRows) {  // the DT stops after this substep
+        if (!D.ctl->error) D.ctl->error = s_reach == kBcOutside ? 4 : 5;
+        D.ctl->more = 0;
+      }
     }
     __syncthreads();
+    if (s_reach > kBcInRows) return;
     const int i_angle = s_angle[0], i_angle2 = s_angle[1];
     const float SigmaMed = D.SigmaMed[1], SigmaMed2 = D.SigmaMed[nrad - 2];
     // Rings 1, 2 and NRAD-2 are read, rings 0, 1 (v_r) and NRAD-1 written: the
     // samples of four sectors are loaded before any is stored.  On a grid so
     // coarse that an offset exceeds a turn, the one wrap of the reference leaves
-    // its target in the next ring, which other sectors read or write: those
-    // offsets keep the sectors in order, one at a time.
+    // its target in another ring, which other sectors read or write: one thread
+    // then takes the sectors in order.
     const int i1 = nsec, iq = (nrad - 2) * nsec, io = (nrad - 1) * nsec;
-    const bool in_ring = abs(i_angle) <= nsec && abs(i_angle2) <= nsec;
-    for (int j = tid; !in_ring && j < nsec; j += kThreads) {
-      int jp = j + i_angle;
-      if (jp >= nsec) jp -= nsec;
-      if (jp < 0) jp += nsec;
+    const bool in_ring = s_reach == kBcInRing;
+    for (int j = 0; !in_ring && tid == 0 && j < nsec; j++) {
+      const int jp = bc_wrap(j, i_angle, nsec), jq = bc_wrap(j, -i_angle2, nsec);
       Dn[jp] = Dn[i1 + j];
       En[jp] = En[i1 + j];
       float Vrad_med = -cs_at(1, j) * (Dn[i1 + j] - SigmaMed) / SigmaMed;
       Vr[i1 + j] = 2. * Vrad_med - Vr[i1 + nsec + j];
-      jp = j - i_angle2;
-      if (jp >= nsec) jp -= nsec;
-      if (jp < 0) jp += nsec;
-      Dn[io + j] = Dn[iq + jp];
-      En[io + j] = En[iq + jp];
+      Dn[io + j] = Dn[iq + jq];
+      En[io + j] = En[iq + jq];
       Vrad_med = cs_at(nrad - 1, j) * (Dn[iq + j] - SigmaMed2) / SigmaMed2;
       Vr[io + j] = 2. * Vrad_med - Vr[iq + j];
     }
@@ -3394,9 +3398,7 @@ __device__ void boundary_edges(const DiskDev& D, float* sm) {
 #pragma unroll
       for (int u = 0; u < 4; u++) {
         const int j = min(j0 + u * kThreads, nsec - 1);
-        int jp = j - i_angle2;
-        if (jp >= nsec) jp -= nsec;
-        if (jp < 0) jp += nsec;
+        const int jp = bc_wrap(j, -i_angle2, nsec);
         d1[u] = Dn[i1 + j];
         e1[u] = En[i1 + j];
         v2[u] = Vr[i1 + nsec + j];
@@ -3411,9 +3413,7 @@ __device__ void boundary_edges(const DiskDev& D, float* sm) {
       for (int u = 0; u < 4; u++) {
         const int j = j0 + u * kThreads;
         if (j >= nsec) break;
-        int jp = j + i_angle;
-        if (jp >= nsec) jp -= nsec;
-        if (jp < 0) jp += nsec;
+        const int jp = bc_wrap(j, i_angle, nsec);
         Dn[jp] = d1[u];
         En[jp] = e1[u];
         float Vrad_med = -c1[u] * (d1[u] - SigmaMed) / SigmaMed;
