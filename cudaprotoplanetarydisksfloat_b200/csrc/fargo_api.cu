@@ -49,7 +49,7 @@ struct fargo_batch {
   DiskDev* d_disks = nullptr;
   DiskCtl* d_ctl = nullptr;
   DiskCtl* h_ctl = nullptr;  // page-locked copy of the control blocks, and a few sums behind it
-  bool retained = false;     // a user of host_copy's rings
+  int retained = 0;          // a user of host_copy's rings
   long long* d_cell_off = nullptr;
   int* d_ring_off = nullptr;
   int4* d_theta = nullptr;
@@ -663,8 +663,7 @@ fargo_status batch_create(fargo_batch* b, int n, const fargo_params* params, con
   CK(cudaMalloc(&b->d_disks, sizeof(DiskDev) * n));
   CK(cudaMalloc(&b->d_ctl, sizeof(DiskCtl) * n));
   CK(cudaMallocHost(&b->h_ctl, sizeof(DiskCtl) * n + sizeof(double) * b->kSums));
-  host_copy_retain();
-  b->retained = true;
+  b->retained = host_copy_retain();
   CK(cudaMemsetAsync(b->d_ctl, 0, sizeof(DiskCtl) * n, b->stream));
   CK(cudaMalloc(&b->d_cell_off, sizeof(long long) * (n + 1)));
   CK(cudaMalloc(&b->d_ring_off, sizeof(int) * (n + 1)));
@@ -762,7 +761,7 @@ void batch_free(fargo_batch* b) {
   for (void* p : ps)
     if (p) cudaFree(p);
   if (b->h_ctl) cudaFreeHost(b->h_ctl);
-  if (b->retained) host_copy_release();
+  if (b->retained) host_copy_release(b->retained);
   if (b->stream) cudaStreamDestroy(b->stream);
 }
 

@@ -5,6 +5,7 @@
 #include <unistd.h>
 
 #include <algorithm>
+#include <atomic>
 #include <condition_variable>
 #include <cstring>
 #include <deque>
@@ -56,12 +57,7 @@ class Ring {
       stop_ = true;
     }
     wake_.notify_all();
-    for (auto& t : threads_) {
-      if (mine())
-        t.join();
-      else
-        t.detach();  // a forked child has the objects but not the threads
-    }
+    for (auto& t : threads_) t.join();
     for (auto& e : ev_)
       if (e) cudaEventDestroy(e);
     if (buf_) cudaFreeHost(buf_);
@@ -109,7 +105,6 @@ class Ring {
     return err;
   }
 
-  bool mine() const { return pid_ == getpid(); }
   std::mutex user;  // held by the copy that uses the ring
 
  private:
@@ -146,16 +141,31 @@ class Ring {
   std::deque<Job> jobs_;
   bool busy_[kSlots] = {};
   bool stop_ = false;
-  const pid_t pid_ = getpid();
 };
 
-// Rings by device.  Plain pointers: what is still open when the process ends
-// is left to the system (its threads and the CUDA context go first).
-std::mutex g_mutex;
-int g_users = 0;
-std::map<int, Ring*>& rings() {
-  static auto* m = new std::map<int, Ring*>();
-  return *m;
+// The rings of one process, by device.  Plain pointers: what is still open when
+// the process ends is left to the system (its threads and the CUDA context go
+// first).
+struct Process {
+  const pid_t pid = getpid();
+  std::mutex m;
+  int users = 0;
+  std::map<int, Ring*> rings;
+};
+std::atomic<Process*> g_process{nullptr};
+
+// This process's own.  A forked child has a copy of the parent's object, whose
+// locks may be held and whose rings' threads are not there: it is never locked
+// nor destroyed, the child makes one of its own.
+Process& process() {
+  const pid_t pid = getpid();
+  Process* p = g_process.load();
+  while (!p || p->pid != pid) {
+    Process* own = new Process();
+    if (g_process.compare_exchange_strong(p, own)) return *own;
+    delete own;
+  }
+  return *p;
 }
 
 // Whether the middle page of the buffer has no memory yet.
@@ -167,30 +177,35 @@ bool fresh(const void* p, size_t bytes) {
 }
 
 Ring* ring_of(int device) {
-  std::lock_guard<std::mutex> l(g_mutex);
-  auto it = rings().find(device);
-  if (it != rings().end()) return it->second;
+  Process& own = process();
+  std::lock_guard<std::mutex> l(own.m);
+  auto it = own.rings.find(device);
+  if (it != own.rings.end()) return it->second;
   Ring* r = new Ring();
   if (!r->open()) {
     delete r;
     r = nullptr;
   }
-  rings()[device] = r;
+  own.rings[device] = r;
   return r;
 }
 
 }  // namespace
 
-void host_copy_retain() {
-  std::lock_guard<std::mutex> l(g_mutex);
-  g_users++;
+int host_copy_retain() {
+  Process& own = process();
+  std::lock_guard<std::mutex> l(own.m);
+  own.users++;
+  return (int)own.pid;
 }
 
-void host_copy_release() {
-  std::lock_guard<std::mutex> l(g_mutex);
-  if (--g_users > 0) return;
-  for (auto& r : rings()) delete r.second;
-  rings().clear();
+void host_copy_release(int user) {
+  if (user != (int)getpid()) return;  // the parent's
+  Process& own = process();
+  std::lock_guard<std::mutex> l(own.m);
+  if (--own.users > 0) return;
+  for (auto& r : own.rings) delete r.second;
+  own.rings.clear();
 }
 
 cudaError_t host_copy(const HostPiece* piece, int n, int device, cudaStream_t stream) {
@@ -201,7 +216,7 @@ cudaError_t host_copy(const HostPiece* piece, int n, int device, cudaStream_t st
   if (through) {
     try {
       Ring* r = ring_of(device);
-      if (r && r->mine()) {
+      if (r) {
         std::unique_lock<std::mutex> l(r->user, std::try_to_lock);
         if (l.owns_lock()) return r->copy(piece, n, total, stream);
       }

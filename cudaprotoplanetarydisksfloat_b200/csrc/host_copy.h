@@ -17,10 +17,12 @@ struct HostPiece {
   size_t bytes;
 };
 
-// One user (a batch) more or less.  The rings and threads are made by the
-// first large copy on a device and given back with the last user.
-void host_copy_retain();
-void host_copy_release();
+// One user (a batch) more or less: host_copy_retain's result goes to
+// host_copy_release.  The rings and threads are made by the first large copy on
+// a device and given back with the last user.  A forked child that drops a batch
+// it inherited leaves the parent's rings alone.
+int host_copy_retain();
+void host_copy_release(int user);
 
 // Copies device memory to host memory behind what the stream holds, and waits
 // for it.  Safe from several threads: while one uses the ring, another's copy

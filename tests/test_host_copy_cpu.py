@@ -1,0 +1,103 @@
+"""The copy ring of csrc/host_copy.cpp without a GPU: the file compiled against a
+few host stand-ins for the runtime's calls.
+
+A forked child that drops what it inherited (a multiprocessing worker whose
+copied object is collected) must return: it has neither the ring's threads nor
+the right to its locks.  The program forks while another thread copies, so that
+locks are held at some of the forks, and gives each child a time limit."""
+import os
+import subprocess
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CSRC = os.path.join(ROOT, "cudaprotoplanetarydisksfloat_b200", "csrc")
+CUDA = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+
+STUBS = r'''
+#include <atomic>
+#include <cstdio>
+#include <cstdlib>
+#include <cstring>
+#include <thread>
+#include <vector>
+#include <sys/wait.h>
+#include <unistd.h>
+#include "host_copy.h"
+
+static std::atomic<long> g_pinned{0};
+extern "C" {
+cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) { *p = std::malloc(n); g_pinned++; return cudaSuccess; }
+cudaError_t cudaFreeHost(void* p) { std::free(p); g_pinned--; return cudaSuccess; }
+cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) { *e = (cudaEvent_t)1; return cudaSuccess; }
+cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
+cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaGetLastError() { return cudaSuccess; }
+cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t) {
+  std::memcpy(d, s, n);
+  return cudaSuccess;
+}
+}
+static std::vector<char> source(size_t n) {
+  std::vector<char> v(n);
+  for (size_t k = 0; k < n; k++) v[k] = (char)(k * 2654435761u >> 13);
+  return v;
+}
+'''
+
+FORK = STUBS + r'''
+int main() {
+  const size_t n = (size_t)30 << 20;
+  const std::vector<char> src = source(n);
+  const int user = host_copy_retain();
+  std::atomic<bool> stop{false};
+  std::atomic<int> bad{0};
+  std::vector<char> first(n);
+  HostPiece p{first.data(), src.data(), n};
+  bad += host_copy(&p, 1, 0, nullptr) != cudaSuccess || first != src;
+  if (g_pinned != 1) return 2;  // the ring was taken
+  std::thread t([&] {
+    std::vector<char> dst(n);
+    while (!stop) {
+      HostPiece q{dst.data(), src.data(), n};
+      bad += host_copy(&q, 1, 0, nullptr) != cudaSuccess || dst != src;
+      const int u = host_copy_retain();
+      host_copy_release(u);
+    }
+  });
+  for (int k = 0; k < 40 && !bad; k++) {
+    const pid_t c = fork();
+    if (c == 0) {
+      alarm(5);  // ends a child that waits for locks or threads it does not have
+      host_copy_release(user);
+      const int u = host_copy_retain();  // and its own use is its own
+      std::vector<char> dst(n);
+      HostPiece q{dst.data(), src.data(), n};
+      const bool ok = host_copy(&q, 1, 0, nullptr) == cudaSuccess && dst == src;
+      host_copy_release(u);
+      _exit(ok ? 0 : 1);
+    }
+    int st = 0;
+    waitpid(c, &st, 0);
+    if (!WIFEXITED(st) || WEXITSTATUS(st)) bad++;
+    usleep(1000);
+  }
+  stop = true;
+  t.join();
+  host_copy_release(user);
+  if (g_pinned != 0) return 3;  // the parent's ring goes with its last user
+  return bad ? 1 : 0;
+}
+'''
+
+
+def _run(tmp_path, text):
+    src, exe = tmp_path / "t.cpp", tmp_path / "t"
+    src.write_text(text)
+    subprocess.check_call(["g++", "-std=c++17", "-O1", "-Wall", "-I" + CSRC, "-I" + os.path.join(CUDA, "include"),
+                           str(src), os.path.join(CSRC, "host_copy.cpp"), "-o", str(exe), "-pthread"])
+    return subprocess.run([str(exe)], timeout=300).returncode
+
+
+def test_forked_child_leaves_the_ring(tmp_path):
+    assert _run(tmp_path, FORK) == 0
