@@ -176,6 +176,15 @@ bool fresh(const void* p, size_t bytes) {
   return mincore(reinterpret_cast<void*>(at), page, &v) == 0 && !(v & 1);
 }
 
+// Ordinary pageable memory.  Anything the runtime knows (page-locked, managed or
+// device memory) it fills itself, by one DMA.
+bool pageable(const void* p) {
+  cudaPointerAttributes a;
+  if (cudaPointerGetAttributes(&a, p) == cudaSuccess) return a.type == cudaMemoryTypeUnregistered;
+  (void)cudaGetLastError();
+  return false;
+}
+
 Ring* ring_of(int device) {
   Process& own = process();
   std::lock_guard<std::mutex> l(own.m);
@@ -213,6 +222,7 @@ cudaError_t host_copy(const HostPiece* piece, int n, int device, cudaStream_t st
   for (int k = 0; k < n; k++) total += piece[k].bytes;
   bool through = total >= kBacked;
   for (int k = 0; k < n && !through && total >= kFresh; k++) through = fresh(piece[k].dst, piece[k].bytes);
+  for (int k = 0; k < n && through; k++) through = pageable(piece[k].dst);
   if (through) {
     try {
       Ring* r = ring_of(device);

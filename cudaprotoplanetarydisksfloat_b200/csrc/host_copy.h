@@ -25,6 +25,6 @@ int host_copy_retain();
 void host_copy_release(int user);
 
 // Copies device memory to host memory behind what the stream holds, and waits
-// for it.  Safe from several threads: while one uses the ring, another's copy
+// for it.  A destination that is not pageable is the driver's to fill.  Safe from several threads: while one uses the ring, another's copy
 // takes the plain path.
 cudaError_t host_copy(const HostPiece* piece, int n, int device, cudaStream_t stream);

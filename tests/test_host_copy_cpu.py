@@ -1,6 +1,9 @@
 """The copy ring of csrc/host_copy.cpp without a GPU: the file compiled against a
 few host stand-ins for the runtime's calls.
 
+A page-locked destination is filled by one copy of the driver's, not by way of
+the ring (a second pass through host memory).
+
 A forked child that drops what it inherited (a multiprocessing worker whose
 copied object is collected) must return: it has neither the ring's threads nor
 the right to its locks.  The program forks while another thread copies, so that
@@ -24,6 +27,8 @@ STUBS = r'''
 #include "host_copy.h"
 
 static std::atomic<long> g_pinned{0};
+static void* g_locked = nullptr;  // a destination that counts as page-locked, and the copies straight into it
+static std::atomic<long> g_straight{0};
 extern "C" {
 cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) { *p = std::malloc(n); g_pinned++; return cudaSuccess; }
 cudaError_t cudaFreeHost(void* p) { std::free(p); g_pinned--; return cudaSuccess; }
@@ -33,7 +38,12 @@ cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
 cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
 cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaGetLastError() { return cudaSuccess; }
+cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void* p) {
+  a->type = p == g_locked ? cudaMemoryTypeHost : cudaMemoryTypeUnregistered;
+  return cudaSuccess;
+}
 cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t) {
+  g_straight += d == g_locked;
   std::memcpy(d, s, n);
   return cudaSuccess;
 }
@@ -91,6 +101,30 @@ int main() {
 '''
 
 
+LOCKED = STUBS + r'''
+int main() {
+  const int user = host_copy_retain();
+  int bad = 0;
+  for (const size_t n : {(size_t)3 << 20, (size_t)30 << 20}) {
+    const std::vector<char> src = source(n);
+    // fresh pages (malloc of this size maps them) and touched ones
+    for (int touched = 0; touched < 2; touched++) {
+      char* dst = (char*)std::malloc(n);
+      if (touched) std::memset(dst, 1, n);
+      g_locked = dst;
+      g_straight = 0;
+      HostPiece p{dst, src.data(), n};
+      bad += host_copy(&p, 1, 0, nullptr) != cudaSuccess || std::memcmp(dst, src.data(), n) != 0;
+      bad += g_straight != 1 || g_pinned != 0;  // one copy into it, no ring made
+      std::free(dst);
+    }
+  }
+  host_copy_release(user);
+  return bad;
+}
+'''
+
+
 def _run(tmp_path, text):
     src, exe = tmp_path / "t.cpp", tmp_path / "t"
     src.write_text(text)
@@ -101,3 +135,7 @@ def _run(tmp_path, text):
 
 def test_forked_child_leaves_the_ring(tmp_path):
     assert _run(tmp_path, FORK) == 0
+
+
+def test_page_locked_destination_takes_no_detour(tmp_path):
+    assert _run(tmp_path, LOCKED) == 0
