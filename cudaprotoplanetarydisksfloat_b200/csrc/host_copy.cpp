@@ -8,7 +8,6 @@
 #include <atomic>
 #include <condition_variable>
 #include <cstring>
-#include <deque>
 #include <map>
 #include <mutex>
 #include <thread>
@@ -94,7 +93,7 @@ class Ring {
       {
         std::lock_guard<std::mutex> l(m_);
         busy_[s] = true;
-        jobs_.push_back(flight[s]);
+        jobs_[given_++ % kSlots] = flight[s];
       }
       wake_.notify_one();
       landed++;
@@ -122,10 +121,9 @@ class Ring {
   void work() {
     std::unique_lock<std::mutex> l(m_);
     for (;;) {
-      wake_.wait(l, [this] { return stop_ || !jobs_.empty(); });
-      if (jobs_.empty()) return;
-      const Job j = jobs_.front();
-      jobs_.pop_front();
+      wake_.wait(l, [this] { return stop_ || taken_ != given_; });
+      if (taken_ == given_) return;
+      const Job j = jobs_[taken_++ % kSlots];
       l.unlock();
       std::memcpy(j.to, j.from, j.bytes);
       l.lock();
@@ -138,7 +136,8 @@ class Ring {
   std::vector<std::thread> threads_;
   std::mutex m_;
   std::condition_variable wake_, done_;
-  std::deque<Job> jobs_;
+  Job jobs_[kSlots];  // at most one per slot: nothing is allocated while copies are in flight
+  unsigned long given_ = 0, taken_ = 0;
   bool busy_[kSlots] = {};
   bool stop_ = false;
 };
@@ -190,12 +189,12 @@ Ring* ring_of(int device) {
   std::lock_guard<std::mutex> l(own.m);
   auto it = own.rings.find(device);
   if (it != own.rings.end()) return it->second;
-  Ring* r = new Ring();
+  Ring*& r = own.rings[device];  // null if it cannot be made
+  r = new Ring();
   if (!r->open()) {
     delete r;
     r = nullptr;
   }
-  own.rings[device] = r;
   return r;
 }
 

@@ -1,6 +1,9 @@
 """The copy ring of csrc/host_copy.cpp without a GPU: the file compiled against a
 few host stand-ins for the runtime's calls.
 
+Once the ring is there, a copy allocates nothing: an exception in the middle of
+one would leave its pieces with the threads, and a slot taken for good.
+
 A page-locked destination is filled by one copy of the driver's, not by way of
 the ring (a second pass through host memory).
 
@@ -125,6 +128,31 @@ int main() {
 '''
 
 
+NO_ALLOC = STUBS + r'''
+static std::atomic<long> g_news{0};
+void* operator new(size_t n) {
+  g_news++;
+  if (void* p = std::malloc(n)) return p;
+  throw std::bad_alloc();
+}
+void operator delete(void* p) noexcept { std::free(p); }
+void operator delete(void* p, size_t) noexcept { std::free(p); }
+int main() {
+  const size_t n = (size_t)70 << 20;  // 70 pieces: every slot several times
+  const std::vector<char> src = source(n);
+  std::vector<char> dst(n);
+  const int user = host_copy_retain();
+  HostPiece p{dst.data(), src.data(), n};
+  int bad = host_copy(&p, 1, 0, nullptr) != cudaSuccess;
+  const long before = g_news;
+  for (int k = 0; k < 5; k++) bad += host_copy(&p, 1, 0, nullptr) != cudaSuccess || dst != src;
+  bad += g_news != before;
+  host_copy_release(user);
+  return bad;
+}
+'''
+
+
 def _run(tmp_path, text):
     src, exe = tmp_path / "t.cpp", tmp_path / "t"
     src.write_text(text)
@@ -139,3 +167,7 @@ def test_forked_child_leaves_the_ring(tmp_path):
 
 def test_page_locked_destination_takes_no_detour(tmp_path):
     assert _run(tmp_path, LOCKED) == 0
+
+
+def test_copies_allocate_nothing(tmp_path):
+    assert _run(tmp_path, NO_ALLOC) == 0
