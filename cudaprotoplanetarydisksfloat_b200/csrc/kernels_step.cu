@@ -74,8 +74,12 @@ constexpr int kThreads = 256;
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // Lets the next kernel of the chain start now.  What that one does before its
-// wait may use only what was complete before this kernel passed its own wait, and
-// reads fields through L2.  Three places, each a few microseconds of serial work
+// wait may use only what was complete before this kernel passed its own wait: the
+// writers had ended then, with their results in L2.  Nothing orders the loads
+// themselves, and an SM that ran none of the kernels in between may hold an older
+// copy in L1, so every field and every word of the control block that is read
+// before the wait is read through L2 (before_wait, the tensor copies, 16-byte
+// cp.async).  Three places, each a few microseconds of serial work
 // that leaves most of the chip idle:
 //  - the ring means of the CFL (one disk): k_cfl_force loads its cells and forms
 //    the disk force, and waits before it reads the ring means;
@@ -89,6 +93,12 @@ __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait
 // batch keeps the waits at the start: its kernels fill the chip by themselves (16
 // disks 313 with any of the three).
 __device__ __forceinline__ void chain_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// A value that another kernel wrote, read ahead of chain_wait (early), else plainly.
+template <bool early, class T>
+__device__ __forceinline__ T before_wait(const T& x) {
+  return early ? __ldcg(&x) : x;
+}
 
 __device__ __forceinline__ int disk_of_cell(const BatchDev& B, long long c) {
   int lo = 0, hi = B.ndisk - 1;
@@ -1114,14 +1124,14 @@ __global__ void __launch_bounds__(kThreads, NB <= 1 ? 3 : 2) k_cfl_force(BatchDe
         __syncthreads();
       }
       const DiskCtl* C = sD.ctl;
-      const int nb = min(C->nbody, NB);
+      const int nb = min(before_wait<solo>(C->nbody), NB);
       if (tid == 0) s_nbody = nb;
       if (tid < nb) {
-        s_b[0][tid] = C->bx[tid];
-        s_b[1][tid] = C->by[tid];
-        s_b[2][tid] = C->brs[tid];
-        s_b[3][tid] = C->brh[tid];
-        s_b[4][tid] = C->ba[tid];
+        s_b[0][tid] = before_wait<solo>(C->bx[tid]);
+        s_b[1][tid] = before_wait<solo>(C->by[tid]);
+        s_b[2][tid] = before_wait<solo>(C->brs[tid]);
+        s_b[3][tid] = before_wait<solo>(C->brh[tid]);
+        s_b[4][tid] = before_wait<solo>(C->ba[tid]);
       }
       __syncthreads();
     }
@@ -1449,7 +1459,7 @@ __global__ void __launch_bounds__(kThreads) k_potential(BatchDev B) {
     y[u] = Rm * sp[u];
     P[u] = 0.0f;
   }
-  const int nb = C->nb;
+  const int nb = before_wait<early>(C->nb);
   const bool ind = D.Indirect_Term;
   auto term = [&](int u, float xp, float yp, float mp, float sm, float ip3) -> float {
     float distance = (x[u] - xp) * (x[u] - xp) + (y[u] - yp) * (y[u] - yp);
@@ -1464,7 +1474,9 @@ __global__ void __launch_bounds__(kThreads) k_potential(BatchDev B) {
 #pragma unroll
     for (int k = 0; k < kEarly; k++) {
       if (k >= nb) break;
-      const float xp = C->pxp[k], yp = C->pyp[k], mp = C->pmass[k], sm = C->psmooth[k], ip3 = C->pipd3[k];
+      const float xp = before_wait<early>(C->pxp[k]), yp = before_wait<early>(C->pyp[k]),
+                  mp = before_wait<early>(C->pmass[k]), sm = before_wait<early>(C->psmooth[k]),
+                  ip3 = before_wait<early>(C->pipd3[k]);
 #pragma unroll
       for (int u = 0; u < 4; u++) pe[k][u] = term(u, xp, yp, mp, sm, ip3);
     }
@@ -2970,6 +2982,8 @@ __global__ void __launch_bounds__(kTT, 2) k_transport(BatchDev B, const int4* __
   constexpr bool early = solo && nq == 5;
   chain_start<solo, early>(B, &sD);
   if (early && B.ragged) chain_wait();
+  // the fields' writers used the generic proxy, the tensor copies read by the async one
+  if (early && p == 0) asm volatile("fence.proxy.async.global;\n" ::: "memory");
   const int nak = solo ? 1 : (nq == 5) ? B.act[1] : B.act[2];
   const int* aoff = (nq == 5) ? B.act_iso_off : B.act_adi_off;
   const int* adisk = (nq == 5) ? B.act_iso_disk : B.act_adi_disk;
@@ -3011,8 +3025,8 @@ __global__ void __launch_bounds__(kTT, 2) k_transport(BatchDev B, const int4* __
     const int nsec = D.nsec, nrad = D.nrad;
     const int nb = min(kBR, nrad - i0);
     const int L = S + 8;
-    const float dt = C->dtf;
-    const float Om = C->OmegaFrame;
+    const float dt = before_wait<early>(C->dtf);
+    const float Om = before_wait<early>(C->OmegaFrame);
     const bool fast = D.FastTransport;
     const float dtheta = 2.0f * (float)PI_D / (float)nsec;
     auto shifts = [&]() {
