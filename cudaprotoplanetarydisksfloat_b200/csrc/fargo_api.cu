@@ -508,9 +508,11 @@ fargo_status build_graph(fargo_batch* b) {
   for (int d = 0; d < (int)b->disks.size(); d++)
     if (b->disks[d].sg) sg_capture_substep(b->disks[d].sg, b->bd, d, &b->disks[d].dev, b->stream);
   if (fork) sg.leave();
-  fargo_launch_substep(b->bd, b->handle, 1, b->stream, b->max_nsec, nullptr, nullptr,
-                       FARGO_PART_HEAD | FARGO_PART_TAIL, fork ? &sg : nullptr);
+  cudaError_t eb = fargo_launch_substep(b->bd, b->handle, 1, b->stream, b->max_nsec, nullptr, nullptr,
+                                        FARGO_PART_HEAD | FARGO_PART_TAIL, fork ? &sg : nullptr);
+  if (eb == cudaSuccess) eb = sg.err;
   cudaError_t ec = cudaStreamEndCapture(b->stream, &body);
+  if (ec == cudaSuccess) ec = eb;
   if (ec != cudaSuccess) return set_err(b, FARGO_ECUDA, "graph capture: %s", cudaGetErrorString(ec));
   CK(cudaGraphInstantiate(&b->exec, b->graph, 0));
   return FARGO_OK;
@@ -784,7 +786,7 @@ fargo_status advance_dt_async(fargo_batch* b) {
     while (more) {
       for (int d = 0; d < (int)b->disks.size(); d++)
         if (b->disks[d].sg) sg_capture_substep(b->disks[d].sg, b->bd, d, &b->disks[d].dev, b->stream);
-      fargo_launch_substep(b->bd, 0, 0, b->stream, b->max_nsec, nullptr);
+      CK(fargo_launch_substep(b->bd, 0, 0, b->stream, b->max_nsec, nullptr));
       CK(cudaMemcpyAsync(hflag, b->d_flags, sizeof(int), cudaMemcpyDeviceToHost, b->stream));
       CK(cudaStreamSynchronize(b->stream));
       more = *hflag;
@@ -1664,7 +1666,7 @@ fargo_status fargo_stripe_forces(fargo_ctx* ctx, double* block) {
   if (!ctx || !ctx->b.stripe || !block) return FARGO_EINVAL;
   fargo_batch* b = &ctx->b;
   CK(cudaSetDevice(b->device));
-  fargo_launch_substep(b->bd, 0, 0, b->stream, b->max_nsec, &b->launches, nullptr, FARGO_PART_HEAD);
+  CK(fargo_launch_substep(b->bd, 0, 0, b->stream, b->max_nsec, &b->launches, nullptr, FARGO_PART_HEAD));
   fargo_launch_stripe_block(b->bd, block, b->stream);
   b->launches += 1;
   CK(cudaGetLastError());
@@ -1678,7 +1680,7 @@ fargo_status fargo_stripe_substep(fargo_ctx* ctx, const double* blocks, int nstr
   if (fargo_launch_stripe_finish(b->bd, blocks, nstripe, stride, b->stream))
     return set_err(b, FARGO_EINVAL, "stripe count %d out of range", nstripe);
   b->launches += 1;
-  fargo_launch_substep(b->bd, 0, 0, b->stream, b->max_nsec, &b->launches, nullptr, FARGO_PART_TAIL);
+  CK(fargo_launch_substep(b->bd, 0, 0, b->stream, b->max_nsec, &b->launches, nullptr, FARGO_PART_TAIL));
   CK(cudaGetLastError());
   return FARGO_OK;
 }

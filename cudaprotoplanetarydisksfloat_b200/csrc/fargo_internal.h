@@ -14,7 +14,6 @@
 //                 potential parameters, force sums, logs.
 #pragma once
 #include <cstdint>
-#include <vector>
 #include <cuda_runtime.h>
 
 #define FARGO_PI 3.14159265358979323844
@@ -208,28 +207,46 @@ struct BatchDev {
 // A side branch of a graph under capture, without a second stream: the nodes
 // launched between begin() and leave() become a branch, those after leave()
 // depend on what preceded begin(), and join() makes the next one depend on the
-// branch too.  begin() is false, and nothing happens, outside a capture.
+// branch too.  begin() is false, and nothing happens, outside a capture.  err:
+// the first call that failed; the graph is then not to be used (a join that adds
+// no edge would leave the branch unordered), and the later calls do nothing.
 struct GraphBranch {
+  static constexpr size_t kMost = 8;  // nodes a branch may begin or end with
+  struct Nodes {
+    cudaGraphNode_t node[kMost];
+    size_t n = 0;
+  };
   cudaStream_t s = nullptr;
-  std::vector<cudaGraphNode_t> before, tip;
-  static bool nodes(cudaStream_t s, std::vector<cudaGraphNode_t>& v) {
+  cudaError_t err = cudaSuccess;
+  Nodes before, tip;
+  bool nodes(Nodes& v) {
     cudaStreamCaptureStatus st;
     const cudaGraphNode_t* deps = nullptr;
     size_t n = 0;
-    if (cudaStreamGetCaptureInfo(s, &st, nullptr, nullptr, &deps, &n) != cudaSuccess) return false;
-    if (st != cudaStreamCaptureStatusActive) return false;
-    v.assign(deps, deps + n);
+    err = cudaStreamGetCaptureInfo(s, &st, nullptr, nullptr, &deps, &n);
+    if (err != cudaSuccess || st == cudaStreamCaptureStatusNone) return false;
+    if (st != cudaStreamCaptureStatusActive || n > kMost) {
+      err = cudaErrorStreamCaptureInvalidated;
+      return false;
+    }
+    for (v.n = 0; v.n < n; v.n++) v.node[v.n] = deps[v.n];
     return true;
   }
   bool begin(cudaStream_t stream) {
     s = stream;
-    return nodes(s, before);
+    return nodes(before);
   }
   void leave() {
-    nodes(s, tip);
-    cudaStreamUpdateCaptureDependencies(s, before.data(), before.size(), cudaStreamSetCaptureDependencies);
+    if (err != cudaSuccess) return;
+    if (nodes(tip))
+      err = cudaStreamUpdateCaptureDependencies(s, before.node, before.n, cudaStreamSetCaptureDependencies);
+    else if (err == cudaSuccess)
+      err = cudaErrorStreamCaptureInvalidated;  // the capture ended inside the branch
   }
-  void join() { cudaStreamUpdateCaptureDependencies(s, tip.data(), tip.size(), cudaStreamAddCaptureDependencies); }
+  void join() {
+    if (err == cudaSuccess)
+      err = cudaStreamUpdateCaptureDependencies(s, tip.node, tip.n, cudaStreamAddCaptureDependencies);
+  }
 };
 
 // kernel entry points (kernels_step.cu), launched by fargo_api.cu
@@ -275,7 +292,8 @@ inline int fargo_red_blocks(long long cells, int most) {  // two cells a thread,
   /* only_disk >= 0: that disk; -1: every disk still inside its DT */                                         \
   void fargo_launch_cs_refresh(const BatchDev& b, int only_disk, cudaStream_t s);                             \
   void fargo_launch_cs_isothermal(const BatchDev& b, int only_disk, cudaStream_t s);                          \
-  void fargo_launch_substep(const BatchDev& b, cudaGraphConditionalHandle h, int use_handle, cudaStream_t s,   \
+  /* the result: what failed in forming the graph's branches (kernel launches: cudaGetLastError) */             \
+  cudaError_t fargo_launch_substep(const BatchDev& b, cudaGraphConditionalHandle h, int use_handle, cudaStream_t s, \
                             int max_nsec, long long* launches, cudaEvent_t* ev = nullptr,                     \
                             int part = FARGO_PART_HEAD | FARGO_PART_TAIL, GraphBranch* sg = nullptr);           \
   /* radial stripes: the stripe's block for the gather (3 + 4 * bodies * own CFL tiles doubles), and the     \

@@ -23,9 +23,10 @@ void fargo_launch_cs_refresh(const BatchDev& b, int only_disk, cudaStream_t s) {
 void fargo_launch_cs_isothermal(const BatchDev& b, int only_disk, cudaStream_t s) {
   FARGO_BY_MODE(b, fargo_launch_cs_isothermal(b, only_disk, s));
 }
-void fargo_launch_substep(const BatchDev& b, cudaGraphConditionalHandle h, int use_handle, cudaStream_t s,
-                          int max_nsec, long long* launches, cudaEvent_t* ev, int part, GraphBranch* sg) {
-  FARGO_BY_MODE(b, fargo_launch_substep(b, h, use_handle, s, max_nsec, launches, ev, part, sg));
+cudaError_t fargo_launch_substep(const BatchDev& b, cudaGraphConditionalHandle h, int use_handle, cudaStream_t s,
+                                 int max_nsec, long long* launches, cudaEvent_t* ev, int part, GraphBranch* sg) {
+  return b.accurate ? fargo_k_nofma::fargo_launch_substep(b, h, use_handle, s, max_nsec, launches, ev, part, sg)
+                    : fargo_k::fargo_launch_substep(b, h, use_handle, s, max_nsec, launches, ev, part, sg);
 }
 void fargo_launch_stripe_block(const BatchDev& b, double* out, cudaStream_t s) {
   FARGO_BY_MODE(b, fargo_launch_stripe_block(b, out, s));

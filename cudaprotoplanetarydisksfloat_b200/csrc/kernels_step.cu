@@ -3892,8 +3892,8 @@ static void launch_transport(const BatchDev& b, int nitems, const int4* items, c
     go(INST(k_transport, nq, 8), grid, kTT, transport_smem_bytes<8>(adi), s, pdl, b, items);
 }
 
-void fargo_launch_substep(const BatchDev& b, cudaGraphConditionalHandle h, int use_handle, cudaStream_t s,
-                          int max_nsec, long long* launches, cudaEvent_t* ev, int part, GraphBranch* sg) {
+cudaError_t fargo_launch_substep(const BatchDev& b, cudaGraphConditionalHandle h, int use_handle, cudaStream_t s,
+                                 int max_nsec, long long* launches, cudaEvent_t* ev, int part, GraphBranch* sg) {
   (void)max_nsec;
   // chained launches, unless each kernel is timed on its own
   const bool pdl = !ev;
@@ -3921,7 +3921,7 @@ void fargo_launch_substep(const BatchDev& b, cudaGraphConditionalHandle h, int u
   }
   if (!(part & FARGO_PART_TAIL)) {
     if (launches) *launches += 2;
-    return;
+    return cudaSuccess;
   }
   REC();
   // a block of the early form has one tile at most (one disk's cells per quad tile)
@@ -3988,6 +3988,7 @@ void fargo_launch_substep(const BatchDev& b, cudaGraphConditionalHandle h, int u
 #undef SRC1
 #undef REC
   if (launches) *launches += FARGO_KNS::fargo_substep_launches(b) - ((part & FARGO_PART_HEAD) ? 0 : 2);
+  return sg && sg->err != cudaSuccess ? sg->err : branch.err != cudaSuccess ? branch.err : heat.err;
 }
 
 void fargo_launch_stripe_block(const BatchDev& b, double* out, cudaStream_t s) {
