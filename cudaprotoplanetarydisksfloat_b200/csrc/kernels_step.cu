@@ -3928,10 +3928,12 @@ cudaError_t fargo_launch_substep(const BatchDev& b, cudaGraphConditionalHandle h
   const bool ahead = solo && (b.ncell + FARGO_QTILE - 1) / FARGO_QTILE <= b.g_potential;
   go((ahead ? k_potential<true, true> : solo ? k_potential<true, false> : k_potential<false, false>), b.g_potential, kThreads, 0, s, pdl && (part & FARGO_PART_HEAD), b);
   REC();
-  // inside a graph the planets run beside the rest of the substep, unless its
-  // kernels read the new frame
+  // in the library's graph the planets run beside the rest of the substep, unless its
+  // kernels read the new frame.  (A caller that captures the stripe calls has the
+  // kernels in line: what it captures next must find them all before it.)
+  const bool own = use_handle != 0;
   GraphBranch branch;
-  const bool fork = !b.any_corot && branch.begin(s);
+  const bool fork = own && !b.any_corot && branch.begin(s);
   go(k_planets, b.ndisk, kThreads, 0, s, false, b);
   if (fork) branch.leave();
   REC();
@@ -3965,7 +3967,7 @@ cudaError_t fargo_launch_substep(const BatchDev& b, cudaGraphConditionalHandle h
   // 256x768 64.5 -> 64.3; behind a boundary call the branch cost more than it
   // gave, 113.9 -> 115.2)
   GraphBranch heat;
-  const bool beside = b.ntheta_adi && !b.any_bc && heat.begin(s);
+  const bool beside = own && b.ntheta_adi && !b.any_bc && heat.begin(s);
   if (b.ntheta_adi) go((solo ? k_energy<true> : k_energy<false>), b.g_energy, kThreads, 0, s, pdl, b);
   if (beside) heat.leave();
   REC();
