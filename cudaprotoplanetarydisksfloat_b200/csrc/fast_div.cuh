@@ -43,11 +43,25 @@ __device__ __forceinline__ double div_by_recip_d(double x, double d, double r) {
 // boundary, and one ulp from it then (tests/test_gpu_division.py counts
 // both).  For normal y and quotient; four instructions against the IEEE
 // sequence's ~ten with its special-case branch.
-//
-// The reciprocal is the flushing form: for a normal y (up to 2^125) it has the
-// bits of rcp.approx.f32, and its product with x those of __fdividef(x, y) (no
-// difference on 4e9 operand pairs), without the instructions by which those
-// handle a subnormal y; a subnormal y would count as zero.
+__device__ __forceinline__ float rcp_approx(float y) {
+  float r;
+  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(y));
+  return r;
+}
+__device__ __forceinline__ float div_refined(float x, float y) {
+  const float r = rcp_approx(y);
+  const float q0 = __fmul_rn(x, r);
+  return __fmaf_rn(__fmaf_rn(-q0, y, x), r, q0);
+}
+
+// The transport's reciprocal is the flushing form: for a normal y (up to 2^126)
+// it has the bits of rcp.approx.f32, and its product with x those of
+// __fdividef(x, y) (no difference on 4e9 operand pairs), without the
+// instructions by which those handle a subnormal y; a subnormal y counts as
+// zero.  No divisor whose quotient the transport uses is subnormal: a slope is
+// used where the product of its two differences is above zero, so at least one
+// of them, and their sum, is above 2^-75; and S + 1e-20f, rounded to at least
+// 2^-91 there, is zero or above that.  (Above 2^126 both forms give zero.)
 __device__ __forceinline__ float rcp_ftz(float y) {
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(y));
@@ -55,7 +69,12 @@ __device__ __forceinline__ float rcp_ftz(float y) {
 }
 // the fast quotient (2 ulp) of normal operands
 __device__ __forceinline__ float div_fast(float x, float y) { return __fmul_rn(x, rcp_ftz(y)); }
-__device__ __forceinline__ float div_refined(float x, float y) {
+// div_refined for a divisor that is zero, infinite or between 2^-126 and 2^126,
+// the same bits: a square root is (2^-75 to 2^64).  Others keep the full range:
+// flushing everywhere (densities, distances cubed) saved 1.4% of a substep
+// (16 disks 317 -> 313 us, 1024x3072 345 -> 340 us) and lost the outer factors of
+// four, where these divisors used to work.
+__device__ __forceinline__ float div_refined_root(float x, float y) {
   const float r = rcp_ftz(y);
   const float q0 = __fmul_rn(x, r);
   return __fmaf_rn(__fmaf_rn(-q0, y, x), r, q0);

@@ -1464,7 +1464,7 @@ __global__ void __launch_bounds__(kThreads) k_potential(BatchDev B) {
   auto term = [&](int u, float xp, float yp, float mp, float sm, float ip3) -> float {
     float distance = (x[u] - xp) * (x[u] - xp) + (y[u] - yp) * (y[u] - yp);
     float distancesmooth = sqrtf(distance + sm);
-    float pot = div_refined(-mp, distancesmooth);  // -G*mplanet/distancesmooth
+    float pot = div_refined_root(-mp, distancesmooth);  // -G*mplanet/distancesmooth
     if (ind) pot += mp * ip3 * (x[u] * xp + y[u] * yp);
     return pot;
   };
