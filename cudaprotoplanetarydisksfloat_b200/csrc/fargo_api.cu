@@ -30,7 +30,8 @@ namespace {
 
 
 struct DiskHost {
-  int seg_out = FARGO_SEG_OUT;  // transport segment width of this disk (autotuned per NSEC class)
+  int seg_tuned = 0;            // transport segment width chosen by the autotuner (0: none)
+  int seg_out = FARGO_SEG_OUT;  // ... and the one in use (build_items)
   fargo_params p;
   fargo_planets planets0;
   HostTables t;
@@ -53,7 +54,6 @@ struct fargo_batch {
   long long* d_cell_off = nullptr;
   int* d_ring_off = nullptr;
   int4* d_theta = nullptr;
-  int seg_out = FARGO_SEG_OUT;  // transport segment width in use (autotuned)
   int* d_flags = nullptr;
   int* d_act = nullptr;  // every compacted-list array in one allocation
   long long* d_act_cell = nullptr;
@@ -518,20 +518,43 @@ fargo_status build_graph(fargo_batch* b) {
   return FARGO_OK;
 }
 
+// A batch whose transport items at FARGO_SEG_NARROW sectors are no more than two
+// per SM is small: every item then runs at once, and an item of the narrow
+// transport takes about two thirds as long as a wide one (128x384: 32 wide items
+// 12.6 us, 64 narrow ones 7.8 us; 256x768 adiabatic 16.9 and 11.4 us).
+bool small_at(const fargo_batch* b, int width) {
+  int nsm = 148;
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, b->device);
+  long long items = 0;
+  for (auto& h : b->disks)
+    items += (long long)((h.p.NRAD + FARGO_BAND - 1) / FARGO_BAND) * ((h.p.NSEC + width - 1) / width);
+  return items <= 2LL * nsm;
+}
+bool small_batch(const fargo_batch* b) { return small_at(b, FARGO_SEG_NARROW); }
+// The one width that the autotuner has for a small batch, whose items run all at
+// once whatever their width and take the same time (96 against 120 sectors: within
+// 1 us a substep on eight grids from 64x192 to 320x700): 96 while that many
+// still do, else 120.
+int narrow_width(const fargo_batch* b) { return small_at(b, 96) ? 96 : FARGO_SEG_NARROW; }
+
 // Segment widths chosen by the autotuner, kept for the life of the process
-// per class of disk (NSEC, adiabatic, precision mode): a batch created later
-// with disks of a tuned class starts from the tuned width.  The transport's
-// results do not depend on the width (its arithmetic is contraction-free and
-// per cell), only its speed does.
-using SegKey = std::tuple<int, int, int>;
+// per class of disk (NSEC, adiabatic, precision mode, in a small batch or not:
+// the widths of the two forms of the transport have nothing to do with each
+// other): a batch created later with disks of a tuned class starts from the
+// tuned width.  The transport's results do not depend on the width (its
+// arithmetic is contraction-free and per cell), only its speed does.
+using SegKey = std::tuple<int, int, int, bool>;
 std::mutex g_seg_mutex;
 std::map<SegKey, int> g_seg_cache;
-SegKey seg_key(const DiskHost& h) { return SegKey(h.p.NSEC, h.p.Adiabatic ? 1 : 0, h.dev.accurate); }
+SegKey seg_key(const DiskHost& h, bool small) {
+  return SegKey(h.p.NSEC, h.p.Adiabatic ? 1 : 0, h.dev.accurate, small);
+}
 void apply_seg_cache(fargo_batch* b) {
+  const bool small = small_batch(b);
   std::lock_guard<std::mutex> lock(g_seg_mutex);
   for (auto& h : b->disks) {
-    auto it = g_seg_cache.find(seg_key(h));
-    if (it != g_seg_cache.end()) h.seg_out = it->second;
+    auto it = g_seg_cache.find(seg_key(h, small));
+    if (it != g_seg_cache.end()) h.seg_tuned = it->second;
   }
 }
 
@@ -539,27 +562,22 @@ void apply_seg_cache(fargo_batch* b) {
 // nseg near-equal azimuthal segments of at most the disk's seg_out source
 // sectors (the sectors a band reads; each ring stores them shifted by its
 // Nshift); isothermal and adiabatic disks in separate lists.  Sets each
-// disk's item0 / nitems (host copy) and returns the widest segment.
-//
-// A batch whose items at FARGO_SEG_NARROW sectors are no more than two per SM
-// takes the narrow transport: every item then runs at once, and a narrow item
-// takes about two thirds as long as a wide one (128x384: 32 wide items 12.6 us, 64
-// narrow ones 7.8 us; 256x768 adiabatic 16.9 and 11.4 us).
+// disk's seg_out, item0 and nitems (host copy) and returns the widest segment.
+// A small batch takes the narrow transport.
 int build_items(fargo_batch* b, std::vector<int4>& theta_iso, std::vector<int4>& theta_adi) {
   int seg_max = 0;
-  int nsm = 148;
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, b->device);
-  long long narrow = 0;
-  for (auto& h : b->disks)
-    narrow += (long long)((h.p.NRAD + FARGO_BAND - 1) / FARGO_BAND) *
-              ((h.p.NSEC + FARGO_SEG_NARROW - 1) / FARGO_SEG_NARROW);
-  b->bd.tr_narrow = narrow <= 2LL * nsm;
+  const bool narrow = small_batch(b);
+  b->bd.tr_narrow = narrow;
   theta_iso.clear();
   theta_adi.clear();
   for (int d = 0; d < (int)b->disks.size(); d++) {
     DiskHost& h = b->disks[d];
     const int nrad = h.p.NRAD, nsec = h.p.NSEC;
-    const int seg_out = b->bd.tr_narrow ? std::min(h.seg_out, FARGO_SEG_NARROW) : h.seg_out;
+    // (a width tuned in a smaller batch must not cost this one a second wave)
+    h.seg_out = !h.seg_tuned ? (narrow ? FARGO_SEG_NARROW : FARGO_SEG_OUT)
+                : narrow     ? std::max(h.seg_tuned, narrow_width(b))
+                             : h.seg_tuned;
+    const int seg_out = h.seg_out;
     std::vector<int4>& theta = h.p.Adiabatic ? theta_adi : theta_iso;
     h.dev.item0 = (int)theta.size();
     const int nseg = (nsec + seg_out - 1) / seg_out;
@@ -1347,7 +1365,9 @@ fargo_status batch_autotune(fargo_batch* b, int reps, int* chosen) {
   if (!b || reps < 1) return FARGO_EINVAL;
   CK(cudaSetDevice(b->device));
   CK(cudaStreamSynchronize(b->stream));
-  static const int cand[] = {96, 128, 160, 192, 224, FARGO_SEG_MAX};
+  const bool small = small_batch(b);
+  std::vector<int> cand = {96, 128, 160, 192, 224, FARGO_SEG_MAX};
+  if (small) cand = {narrow_width(b)};
   cudaEvent_t e0, e1;
   CK(cudaEventCreate(&e0));
   CK(cudaEventCreate(&e1));
@@ -1369,20 +1389,20 @@ fargo_status batch_autotune(fargo_batch* b, int reps, int* chosen) {
   };
   // the classes of disk, largest share of cells first
   std::map<SegKey, long long> cells;
-  for (auto& h : b->disks) cells[seg_key(h)] += (long long)h.p.NRAD * h.p.NSEC;
+  for (auto& h : b->disks) cells[seg_key(h, small)] += (long long)h.p.NRAD * h.p.NSEC;
   std::vector<std::pair<long long, SegKey>> classes;
   for (auto& kv : cells) classes.push_back({kv.second, kv.first});
   std::sort(classes.begin(), classes.end(), [](const auto& x, const auto& y) { return x.first > y.first; });
   auto set_class = [&](const SegKey& k, int w) {
     for (auto& h : b->disks)
-      if (seg_key(h) == k) h.seg_out = w;
+      if (seg_key(h, small) == k) h.seg_tuned = w;
   };
   // one width for every disk, then each class in turn with the others fixed
   float best_ms = 1e30f;
-  int best = FARGO_SEG_OUT;
+  int best = cand[0];
   fargo_status st = FARGO_OK;
   for (int c : cand) {
-    for (auto& h : b->disks) h.seg_out = c;
+    for (auto& h : b->disks) h.seg_tuned = c;
     float ms = 0.0f;
     if ((st = timed(&ms))) return st;
     if (ms < best_ms) {
@@ -1390,7 +1410,7 @@ fargo_status batch_autotune(fargo_batch* b, int reps, int* chosen) {
       best = c;
     }
   }
-  for (auto& h : b->disks) h.seg_out = best;
+  for (auto& h : b->disks) h.seg_tuned = best;
   if (classes.size() > 1) {
     for (auto& cl : classes) {
       int keep = best;
@@ -1412,12 +1432,11 @@ fargo_status batch_autotune(fargo_batch* b, int reps, int* chosen) {
   if ((st = install_items(b))) return st;
   {
     std::lock_guard<std::mutex> lock(g_seg_mutex);
-    for (auto& h : b->disks) g_seg_cache[seg_key(h)] = h.seg_out;
+    for (auto& h : b->disks) g_seg_cache[seg_key(h, small)] = h.seg_tuned;
   }
-  b->seg_out = best;
   if (chosen) {  // the width of the class with the most cells
     for (auto& h : b->disks)
-      if (seg_key(h) == classes[0].second) *chosen = h.seg_out;
+      if (seg_key(h, small) == classes[0].second) *chosen = h.seg_out;
   }
   return build_graph(b);
 }

@@ -320,12 +320,15 @@ fargo_status fargo_batch_set_precision(fargo_batch* b, int mode);
 /* (new) Tile autotuner: times the transport kernels on the current state for
    azimuthal segment widths 96..244 sectors, first one width for every disk,
    then each class of disk (NSEC, adiabatic, precision mode; largest share of
-   cells first) in turn with the others fixed, and keeps the fastest.
+   cells first) in turn with the others fixed, and keeps the fastest.  A batch
+   of at most two work items per SM at 120 sectors runs a narrower form of the
+   kernel, tuned or not, and has one width to choose from (96, or 120).
    *seg_out: the width of the class with the most cells.  The widths are kept
-   for the life of the process per class: batches created later (and a change
-   of precision mode) start from them.  Results do not depend on the widths.
-   Call between DTs; the state is not advanced.  fargo_batch_segments gives
-   each disk's width (cap entries). */
+   for the life of the process per class, apart for such small batches:
+   batches created later (and a change of precision mode) start from them.
+   Results do not depend on the widths.  Call between DTs; the state is not
+   advanced.  fargo_batch_segments gives the width in use for each disk (cap
+   entries), tuned or not. */
 fargo_status fargo_batch_autotune(fargo_batch* b, int reps, int* seg_out);
 fargo_status fargo_autotune(fargo_ctx* ctx, int reps, int* seg_out);
 fargo_status fargo_batch_segments(fargo_batch* b, int cap, int* seg_per_disk);
