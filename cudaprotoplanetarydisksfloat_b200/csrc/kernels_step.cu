@@ -2314,7 +2314,12 @@ __device__ __forceinline__ void rad_march_s(const TrView& V, const float* sIn, i
     // slope at row i+1.  The isothermal form's last ring of a band takes the outermost
     // row's density quotient unrounded: no other expression needs it there, and
     // the results of earlier builds, in which the compiler contracted just this
-    // product, stay what they were.
+    // product, stay what they were.  The next band takes it rounded, so the
+    // mass that leaves a band and the mass that enters the next one may differ:
+    // the density quotient is 1 within a rounding, its slope therefore a rounding
+    // per ring, and the difference at most a rounding of the mass that crosses the
+    // edge in the substep, itself less than half a ring's by the CFL condition
+    // (tests/test_gpu_mass.py).
     if (nq == 5 && k == NR - 1 && tail)
       rad_slopes<nq, true>(V, i + 1, R1, R2, R3, G2, gs2);
     else
