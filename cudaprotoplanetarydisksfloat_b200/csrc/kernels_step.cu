@@ -493,7 +493,7 @@ __device__ __forceinline__ void copy_words(void* dst, const void* src, int bytes
 // inside its DT), and its DiskDev, constant during a DT, is copied to shared
 // memory before the wait for the previous kernel, so that what is left after the
 // wait are the fields themselves, not a chain of four dependent loads (64x192:
-// 58.2 -> 56.0 us a substep, 256x768 adiabatic 72.7 -> 71.2; as a run-time choice in one
+// 55.0 -> 52.6 us a substep, 256x768 adiabatic 73.5 -> 70.2; as a run-time choice in one
 // instance it cost the 16-disk sweep 1.5%).
 // late (with solo): the caller waits later, on every path.
 template <bool solo, bool late = false>
